@@ -87,6 +87,25 @@ void launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, std::size_t
     check(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...), what);
 }
 
+/// The same in clusters of `cluster` consecutive blocks (the grid a multiple of it).
+template <class... Params, class... Args>
+void launch_cluster_kernel(void (*kernel)(Params...), unsigned cluster, dim3 grid, dim3 block, std::size_t smem, cudaStream_t stream, const char* what, Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = launch_overlap() ? 2 : 1;
+    check(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...), what);
+}
+
 /// Default scratch size: two 128 x 256 float32 tiles for each of `sm_count` CTAs.
 std::size_t default_workspace_bytes(int sm_count);
 

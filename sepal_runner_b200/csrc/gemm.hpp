@@ -44,6 +44,7 @@ inline constexpr std::size_t kGroup = 128;  // values of k per int8 scale (the r
 ///       operand, widened and scaled into tensor memory, the tokens the second, w of them to a tile of 256 weight rows (256 and 320: two
 ///       blocks of 128 and 160 that share the converted weights); whole tiles. -1 picks it, and w, by an estimate of both families
 ///       (pick_w8t_tokens in gemm_tc.cu).
+///   1024 + s, 1024 + 16 + s (s 1 .. 8, at most 256 rows): the few-rows kernel (gemm_few.cu), a tile's k in s parts, two CTAs or one to an SM.
 inline constexpr int kConfigs = 4;
 
 /// Row of the stacked [gate; up] matrix that packed row p holds (the reference's pack_gate_up_source,

@@ -119,10 +119,13 @@ def pack_gate_up_source(p: int, inter: int) -> int:
 
 
 def _stream_ptr(stream) -> int:
+    """The cudaStream_t of `stream`, or of the current stream. Asked for as a number: torch.cuda.current_stream() builds a Stream object
+    first, which costs a launcher more host time (3.3 us) than the launch itself."""
+    if stream is not None:
+        return int(stream.cuda_stream)
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return int(s.cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 @dataclass
