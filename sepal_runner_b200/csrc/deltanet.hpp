@@ -9,8 +9,8 @@
 //
 // State. A request owns a slot: its recurrent state [value heads, dk, dv] float32 and the last K - 1 rows of `mixed`. A call holds runs
 // of consecutive tokens of different requests; a run continues its slot's state and leaves it updated, so a request cut into several
-// calls gives what it gives in one. The scan takes a run in chunks of sixteen tokens (eight warps per run and value head, each with 16
-// columns of the float32 state in registers; the chunk's matrix products on the tensor cores with TF32 operands).
+// calls gives what it gives in one. The scan takes a run in chunks of sixteen tokens (warps that each hold 64 rows by 16 columns of the
+// float32 state in registers; the chunk's matrix products on the tensor cores with TF32 operands).
 #pragma once
 
 #include <cstddef>
@@ -49,15 +49,13 @@ struct DeltaNetWeights {
 };
 
 /// Scratch of one call (device, float32, 16-byte aligned), sized for the call's tokens N: kq [key_heads, N, 264] (a token's k, q and 8
-/// floats of padding per key head); v, reads [N, value_dim]; coef [value_heads, N, 56] (the chunk coefficients); decay, beta
-/// [N, value_heads].
+/// floats of padding per key head); v, reads [N, value_dim]; coef [value_heads, N, 56] (the chunk coefficients); 2 N value_heads more that
+/// nothing uses.
 struct DeltaNetScratch {
     float* kq = nullptr;
     float* v = nullptr;
     float* reads = nullptr;
     float* coef = nullptr;
-    float* decay = nullptr;
-    float* beta = nullptr;
 };
 
 /// Floats of scratch a call of `tokens` tokens needs, and the scratch carved out of one such allocation.
@@ -70,12 +68,10 @@ inline DeltaNetScratch deltanet_scratch(float* base, const DeltaNetShape& s, std
     sc.v = sc.kq + tokens * s.key_heads * 264;
     sc.reads = sc.v + tokens * s.value_dim();
     sc.coef = sc.reads + tokens * s.value_dim();
-    sc.decay = sc.coef + tokens * s.value_heads * 56;
-    sc.beta = sc.decay + tokens * s.value_heads;
     return sc;
 }
 
-/// The launches of a layer (prepare, tail, chunk coefficients, scan, gated norm). mixed [N, conv_dim], z [N, value_dim], b and a [N, value_heads] are bands of the in-projection's output;
+/// The launches of a layer (prepare with the chunk coefficients, scan, gated norm with the tails). mixed [N, conv_dim], z [N, value_dim], b and a [N, value_heads] are bands of the in-projection's output;
 /// states float32 [slots, value_heads, head_dim, head_dim] and tails float32 [slots, K - 1, conv_dim], both updated in place; out
 /// binary16 [N, value_dim] with row stride out_stride.
 /// `rows` is a HOST array sorted by q_begin.

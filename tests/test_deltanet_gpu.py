@@ -109,6 +109,51 @@ def test_strong_decay(ctx):
     run_case(ctx, key_heads=2, value_heads=heads, taps=4, requests=[(1, 0), (5, 12), (16, 1), (33, 37)], seed=9, half=True, a_log=a_log)
 
 
+def test_more_runs_than_travel_with_the_launch(ctx):
+    """65 and more runs take their table through device memory, up to 64 with the launch; one, three and eight value heads to a key head."""
+    run_case(ctx, key_heads=1, value_heads=1, taps=4, requests=[(1 + i % 19, 1 + i % 3) for i in range(65)], seed=10, half=True)
+    run_case(ctx, key_heads=2, value_heads=6, taps=4, requests=[(1 + 7 * i % 40, 0) for i in range(64)], seed=11, half=True)
+    run_case(ctx, key_heads=1, value_heads=8, taps=2, requests=[(35, 18)], seed=12, half=True)
+
+
+@pytest.mark.parametrize("value_heads,runs,length", [(4, 1, 100), (16, 2, 33), (32, 2, 49)])
+def test_layouts_agree(ctx, value_heads, runs, length):
+    """Bands at odd columns (channel by channel, value by value) give the bits of the same bands at aligned addresses (pairs, fours), whether a
+    block of the scan holds 16 columns of the state or more; tokens between the runs stay as they were."""
+    import torch
+
+    import sepal_runner_b200 as sb
+
+    key_heads, dim = 4, 128
+    shape = sb.DeltaNetShape(key_heads=key_heads, value_heads=value_heads, head_dim=dim, conv_kernel=4, eps=1e-6)
+    vd, cd = value_heads * dim, (2 * key_heads + value_heads) * dim
+    gen = torch.Generator(device="cuda").manual_seed(value_heads)
+    normal = lambda *s: torch.randn(s, generator=gen, device="cuda")  # noqa: E731
+    tokens = runs * (length + 3)
+    rows = [(i * (length + 3) + 1, length, i, i % 2) for i in range(runs)]
+    conv, a_log, dt_bias, norm = normal(cd, 4) * 0.5, normal(value_heads), normal(value_heads), 1 + normal(dim) * 0.1
+    states, tails = normal(runs, value_heads, dim, dim) * 0.05, normal(runs, 3, cd)
+    wide = [normal(tokens, w).half() for w in (cd, vd, value_heads, value_heads)]
+    got = []
+    for shift in (0, 1):
+        bands = [torch.zeros((tokens, w.shape[1] + 7 + shift), dtype=torch.float16, device="cuda")[:, shift:shift + w.shape[1]] if shift else w for w in wide]
+        if shift:
+            for b, w in zip(bands, wide):
+                b.copy_(w)
+        out = torch.full((tokens, vd + shift), 7.0, dtype=torch.float16, device="cuda")[:, shift:]
+        st, tl = states.clone(), tails.clone()
+        keep = sb.deltanet(ctx, shape, rows, *bands, conv, a_log, dt_bias, norm, st, tl, out)
+        ctx.check_status()
+        del keep
+        got.append((out.clone(), st, tl))
+    for a, b in zip(*got):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
+    live = torch.zeros(tokens, dtype=torch.bool)
+    for q_begin, n, _, _ in rows:
+        live[q_begin:q_begin + n] = True
+    assert (got[0][0][~live.cuda()] == 7.0).all()
+
+
 def test_arguments_are_checked(ctx):
     import torch
 
