@@ -1,6 +1,7 @@
 #include "attention.hpp"
 
 #include <algorithm>
+#include <cstring>
 #include <cmath>
 #include <stdexcept>
 #include <string>
@@ -39,12 +40,17 @@ __device__ __forceinline__ bool wait_barrier(uint32_t bar, uint32_t parity, vola
 
 // ---- prepare --------------------------------------------------------------------------------------------------------------------
 
+// Rows of a call, and blocks of an attention launch, whose tables travel with the kernels' parameters: a copy to the device before each
+// launch costs a few microseconds of a short call and keeps the launch from overlapping with the one before it.
+constexpr unsigned kInlineRows = 64, kInlineBlocks = 160;
+
 struct PrepareParams {
-    const AttentionRow* rows;
+    const AttentionRow* far_rows;  // null: the rows below
+    AttentionRow near_rows[kInlineRows];
+    double inv_freq[128];          // theta^(-2 i / rotary_dims), i < rotary_dims / 2
     unsigned n_rows;
-    unsigned heads, kv_heads, head_dim, rotary_dims;
+    unsigned heads, kv_heads, rotary_dims;
     float eps;
-    const double* inv_freq;  // theta^(-2 i / rotary_dims), i < rotary_dims / 2
     const void* q_gate;
     const void* k;
     const void* v;
@@ -65,9 +71,13 @@ __device__ __forceinline__ float band_value(const void* base, unsigned long long
 // One block per token; a warp takes heads in turn (query heads, then key heads, then the value heads' copy). Lane l holds dimensions
 // l, l + 32, ... of the head. Sum of squares: each lane in that order, then a butterfly: fixed, a function of the head alone. The
 // normed head goes through shared memory so that a rotated dimension can read its partner (i with i + rotary_dims / 2) from any lane.
-__global__ void __launch_bounds__(256) attention_prepare_kernel(const PrepareParams p) {
-    __shared__ float cs[256];          // cos then sin of the token's rotary_dims / 2 angles
-    __shared__ float normed[8][256];   // one head per warp
+// What bounds it is the chain load - sum - store of a warp's heads one after the other, so the next head's values are on their way while
+// this one is worked on, and the first head's while the token's angles are formed.
+template <int D>
+__global__ void __launch_bounds__(256) attention_prepare_kernel(const __grid_constant__ PrepareParams p) {
+    constexpr int kPerLane = D / 32;
+    __shared__ float cs[256];        // cos then sin of the token's rotary_dims / 2 angles
+    __shared__ float normed[8][D];   // one head per warp
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
     const unsigned token = blockIdx.x;
@@ -75,11 +85,25 @@ __global__ void __launch_bounds__(256) attention_prepare_kernel(const PreparePar
     unsigned lo = 0, hi = p.n_rows;
     while (hi - lo > 1) {
         const unsigned mid = (lo + hi) / 2;
-        if (p.rows[mid].q_begin <= token) lo = mid; else hi = mid;
+        if ((p.far_rows != nullptr ? p.far_rows[mid].q_begin : p.near_rows[mid].q_begin) <= token) lo = mid; else hi = mid;
     }
-    const AttentionRow row = p.rows[lo];
+    const AttentionRow row = p.far_rows != nullptr ? p.far_rows[lo] : p.near_rows[lo];
     if (token < row.q_begin || token >= row.q_begin + row.length) return;  // a token outside every run (gaps are allowed)
     const unsigned t = token - row.q_begin;
+    const unsigned warp = threadIdx.x / 32, lane = threadIdx.x % 32, warps = blockDim.x / 32;
+    const unsigned jobs = p.heads + 2 * p.kv_heads;
+    const size_t arena_row = (static_cast<size_t>(row.kv_begin) + row.context + t) * (p.kv_heads * D);
+    const auto fetch = [&](unsigned job, float (&x)[kPerLane]) {
+        const void* base = job < p.heads ? p.q_gate : job < p.heads + p.kv_heads ? p.k : p.v;
+        const unsigned half = job < p.heads ? p.q_gate_half : job < p.heads + p.kv_heads ? p.k_half : p.v_half;
+        const size_t at = job < p.heads                ? token * p.q_gate_stride + static_cast<size_t>(job) * 2 * D
+                          : job < p.heads + p.kv_heads ? token * p.k_stride + (job - p.heads) * D
+                                                       : token * p.v_stride + (job - p.heads - p.kv_heads) * D;
+#pragma unroll
+        for (int e = 0; e < kPerLane; ++e) x[e] = band_value(base, at + lane + 32 * e, half);
+    };
+    float x[kPerLane], next[kPerLane];
+    if (warp < jobs) fetch(warp, next);
     const double position = static_cast<double>(row.context + t);
     const unsigned half_rot = p.rotary_dims / 2;
     for (unsigned i = threadIdx.x; i < half_rot; i += blockDim.x) {
@@ -88,38 +112,39 @@ __global__ void __launch_bounds__(256) attention_prepare_kernel(const PreparePar
         cs[128 + i] = static_cast<float>(sin(angle));
     }
     __syncthreads();
-    const unsigned warp = threadIdx.x / 32, lane = threadIdx.x % 32, warps = blockDim.x / 32;
-    const unsigned hd = p.head_dim, per_lane = hd / 32;  // 4 or 8
-    const size_t arena_row = static_cast<size_t>(row.kv_begin) + row.context + t;
-    for (unsigned job = warp; job < p.heads + 2 * p.kv_heads; job += warps) {
+    for (unsigned job = warp; job < jobs; job += warps) {
+#pragma unroll
+        for (int e = 0; e < kPerLane; ++e) x[e] = next[e];
+        if (job + warps < jobs) fetch(job + warps, next);
         if (job >= p.heads + p.kv_heads) {  // a value head: stored as it is
-            const unsigned h = job - p.heads - p.kv_heads;
-            for (unsigned e = 0; e < per_lane; ++e) {
-                const unsigned d = lane + 32 * e;
-                p.v_arena[arena_row * (p.kv_heads * hd) + h * hd + d] = __float2half_rn(band_value(p.v, token * p.v_stride + h * hd + d, p.v_half));
-            }
+            __half* dst = p.v_arena + arena_row + (job - p.heads - p.kv_heads) * D;
+#pragma unroll
+            for (int e = 0; e < kPerLane; ++e) dst[lane + 32 * e] = __float2half_rn(x[e]);
             continue;
         }
         const bool is_q = job < p.heads;
-        const unsigned h = is_q ? job : job - p.heads;
         const float* w = is_q ? p.q_norm : p.k_norm;
-        float x[8];
+        float gain[kPerLane];
         float ss = 0.0f;
-        for (unsigned e = 0; e < per_lane; ++e) {
-            const unsigned d = lane + 32 * e;
-            x[e] = is_q ? band_value(p.q_gate, token * p.q_gate_stride + static_cast<size_t>(h) * 2 * hd + d, p.q_gate_half)
-                        : band_value(p.k, token * p.k_stride + h * hd + d, p.k_half);
+#pragma unroll
+        for (int e = 0; e < kPerLane; ++e) {
+            gain[e] = w[lane + 32 * e];
             ss = __fmaf_rn(x[e], x[e], ss);
         }
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-        const float rms = __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, static_cast<float>(hd)), p.eps));
+        const float rms = __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, static_cast<float>(D)), p.eps));
         __syncwarp();  // the previous head's readers are done with the buffer
-        for (unsigned e = 0; e < per_lane; ++e) normed[warp][lane + 32 * e] = __fmul_rn(__fdiv_rn(x[e], rms), __fadd_rn(1.0f, w[lane + 32 * e]));
+#pragma unroll
+        for (int e = 0; e < kPerLane; ++e) {
+            x[e] = __fmul_rn(__fdiv_rn(x[e], rms), __fadd_rn(1.0f, gain[e]));
+            normed[warp][lane + 32 * e] = x[e];
+        }
         __syncwarp();
-        __half* dst = is_q ? p.q_out + token * p.q_stride + static_cast<size_t>(h) * hd : p.k_arena + arena_row * (p.kv_heads * hd) + h * hd;
-        for (unsigned e = 0; e < per_lane; ++e) {
+        __half* dst = is_q ? p.q_out + token * p.q_stride + static_cast<size_t>(job) * D : p.k_arena + arena_row + (job - p.heads) * D;
+#pragma unroll
+        for (int e = 0; e < kPerLane; ++e) {
             const unsigned d = lane + 32 * e;
-            float y = normed[warp][d];
+            float y = x[e];
             if (d < half_rot) {  // (a, b) -> (a cos - b sin, b cos + a sin) for a = dimension i, b = dimension i + rotary_dims / 2
                 y = __fsub_rn(__fmul_rn(y, cs[d]), __fmul_rn(normed[warp][d + half_rot], cs[128 + d]));
             } else if (d < 2 * half_rot) {
@@ -141,8 +166,10 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 struct AttentionParams {
-    const AttentionRow* rows;
-    const unsigned* blocks;  // (row, query block) pairs, heaviest first
+    const AttentionRow* far_rows;  // null: the tables below
+    const unsigned* far_blocks;    // (row, query block) pairs, heaviest first
+    AttentionRow near_rows[kInlineRows];
+    unsigned near_blocks[2 * kInlineBlocks];
     unsigned heads, group;   // query heads; heads / kv_heads
     float scale_log2;        // log2(e) / sqrt(head_dim)
     const void* gate;
@@ -173,7 +200,7 @@ struct AttentionTile {
 template <int D>
 __global__ void __launch_bounds__(320, 1)
 attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                 const AttentionParams p) {
+                 const __grid_constant__ AttentionParams p) {
     using T = AttentionTile<D>;
     constexpr int kKeys = T::kKeys;
     extern __shared__ uint8_t smem_raw[];
@@ -200,8 +227,8 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
     const unsigned warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const unsigned head = blockIdx.y, kv_head = head / p.group;
-    const AttentionRow row = p.rows[p.blocks[2 * blockIdx.x]];
-    const unsigned qb = p.blocks[2 * blockIdx.x + 1];
+    const AttentionRow row = p.far_rows != nullptr ? p.far_rows[p.far_blocks[2 * blockIdx.x]] : p.near_rows[p.near_blocks[2 * blockIdx.x]];
+    const unsigned qb = p.far_rows != nullptr ? p.far_blocks[2 * blockIdx.x + 1] : p.near_blocks[2 * blockIdx.x + 1];
     const unsigned q0 = qb * kQueries;                                  // first query of the block inside the run
     const unsigned valid = min(static_cast<unsigned>(kQueries), row.length - q0);
     // keys the block's last valid query sees, and the blocks that hold them
@@ -467,7 +494,7 @@ struct AttentionPairTile {
 template <int D>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kAttentionPairThreads, 1)
 attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                      const AttentionParams p) {
+                      const __grid_constant__ AttentionParams p) {
     using T = AttentionPairTile<D>;
     constexpr int kKeys = T::kKeys, kStages = T::kStages;
     extern __shared__ uint8_t smem_raw[];
@@ -493,8 +520,8 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const unsigned rank = ptx::cluster_ctarank();
     const unsigned head = blockIdx.y, kv_head = head / p.group;
     const unsigned block = blockIdx.x / 2;
-    const AttentionRow row = p.rows[p.blocks[2 * block]];
-    const unsigned qb = p.blocks[2 * block + 1];
+    const AttentionRow row = p.far_rows != nullptr ? p.far_rows[p.far_blocks[2 * block]] : p.near_rows[p.near_blocks[2 * block]];
+    const unsigned qb = p.far_rows != nullptr ? p.far_blocks[2 * block + 1] : p.near_blocks[2 * block + 1];
     const unsigned pair_q0 = qb * 2 * kQueries;                         // first query of the pair inside the run
     const unsigned q0 = pair_q0 + rank * kQueries;                      // and of this CTA
     const unsigned pair_valid = min(2u * kQueries, row.length - pair_q0);
@@ -738,21 +765,12 @@ void check_shape(const AttentionShape& s) {
         throw std::invalid_argument("sepal_b200 attention: head_dim must be 128 or 256, heads a multiple of kv_heads, rotary_dims even and at most head_dim");
 }
 
-// The rows and, after them, what else a launch needs, copied to the context's table. Returns the device address of the rows.
-const AttentionRow* upload_rows(Context& ctx, const AttentionRow* rows, std::size_t n_rows, const void* extra, std::size_t extra_bytes, const void** extra_dev,
-                                cudaStream_t stream) {
+// The device memory for a launch's tables of `bytes` bytes: two halves of the context's used in turn, so that the tables of the launch
+// before this one are not overwritten while it may still run. Null when the tables travel with the kernel's parameters (`near`).
+char* table_memory(Context& ctx, std::size_t n_rows, std::size_t bytes, bool near) {
     if (ctx.table == nullptr) throw std::invalid_argument("sepal_b200 attention: this context has no table memory");
-    const std::size_t row_bytes = n_rows * sizeof(AttentionRow);
-    const std::size_t need = (row_bytes + 15) / 16 * 16 + extra_bytes;
-    if (need > ctx.table_bytes / 2) throw std::invalid_argument("sepal_b200 attention: " + std::to_string(n_rows) + " rows are more than the context's table holds");
-    // two halves used in turn, so that the table of the launch before this one is not overwritten while it may still run
-    char* base = static_cast<char*>(ctx.table) + (ctx.table_turn++ & 1u) * (ctx.table_bytes / 2);
-    check(cudaMemcpyAsync(base, rows, row_bytes, cudaMemcpyHostToDevice, stream), "cudaMemcpyAsync(rows)");
-    if (extra_bytes != 0) {
-        check(cudaMemcpyAsync(base + (row_bytes + 15) / 16 * 16, extra, extra_bytes, cudaMemcpyHostToDevice, stream), "cudaMemcpyAsync(table)");
-        *extra_dev = base + (row_bytes + 15) / 16 * 16;
-    }
-    return reinterpret_cast<const AttentionRow*>(base);
+    if (bytes > ctx.table_bytes / 2) throw std::invalid_argument("sepal_b200 attention: " + std::to_string(n_rows) + " rows are more than the context's table holds");
+    return near ? nullptr : static_cast<char*>(ctx.table) + (ctx.table_turn++ & 1u) * (ctx.table_bytes / 2);
 }
 
 void check_rows(const AttentionRow* rows, std::size_t n_rows, std::size_t n_tokens, std::size_t arena_tokens) {
@@ -783,18 +801,21 @@ void launch_attention_prepare(Context& ctx, const AttentionShape& shape, const A
         throw std::invalid_argument("sepal_b200 attention: null pointer");
     check_rows(rows, n_rows, 0, arena_tokens);
     check(cudaSetDevice(ctx.device), "cudaSetDevice");
-    std::vector<double> inv_freq(shape.rotary_dims / 2);
-    for (std::size_t i = 0; i < inv_freq.size(); ++i) inv_freq[i] = std::pow(shape.rope_theta, -static_cast<double>(2 * i) / static_cast<double>(shape.rotary_dims));
-    const void* inv_dev = nullptr;
     PrepareParams p{};
-    p.rows = upload_rows(ctx, rows, n_rows, inv_freq.data(), inv_freq.size() * sizeof(double), &inv_dev, stream);
+    for (std::size_t i = 0; i < shape.rotary_dims / 2; ++i) p.inv_freq[i] = std::pow(shape.rope_theta, -static_cast<double>(2 * i) / static_cast<double>(shape.rotary_dims));
+    const std::size_t row_bytes = n_rows * sizeof(AttentionRow);
+    char* table = table_memory(ctx, n_rows, (row_bytes + 15) / 16 * 16 + shape.rotary_dims / 2 * sizeof(double), n_rows <= kInlineRows);
+    if (table == nullptr) {
+        std::memcpy(p.near_rows, rows, row_bytes);
+    } else {
+        check(cudaMemcpyAsync(table, rows, row_bytes, cudaMemcpyHostToDevice, stream), "cudaMemcpyAsync(rows)");
+        p.far_rows = reinterpret_cast<const AttentionRow*>(table);
+    }
     p.n_rows = static_cast<unsigned>(n_rows);
     p.heads = shape.heads;
     p.kv_heads = shape.kv_heads;
-    p.head_dim = shape.head_dim;
     p.rotary_dims = shape.rotary_dims;
     p.eps = shape.eps;
-    p.inv_freq = static_cast<const double*>(inv_dev);
     p.q_gate = q_gate.data;
     p.k = k.data;
     p.v = v.data;
@@ -812,7 +833,7 @@ void launch_attention_prepare(Context& ctx, const AttentionShape& shape, const A
     p.v_arena = static_cast<__half*>(v_arena);
     const unsigned first = rows[0].q_begin, last = rows[n_rows - 1].q_begin + rows[n_rows - 1].length;
     (void)first;
-    launch_kernel(attention_prepare_kernel, dim3(last), dim3(256), 0, stream, "attention_prepare_kernel launch", p);
+    launch_kernel(shape.head_dim == 128 ? attention_prepare_kernel<128> : attention_prepare_kernel<256>, dim3(last), dim3(256), 0, stream, "attention_prepare_kernel launch", p);
     count_launch();
 }
 
@@ -847,10 +868,18 @@ void launch_attention(Context& ctx, const AttentionShape& shape, const Attention
         table[2 * i] = blocks[i].row;
         table[2 * i + 1] = blocks[i].qb;
     }
-    const void* table_dev = nullptr;
     AttentionParams p{};
-    p.rows = upload_rows(ctx, rows, n_rows, table.data(), table.size() * sizeof(unsigned), &table_dev, stream);
-    p.blocks = static_cast<const unsigned*>(table_dev);
+    const std::size_t row_bytes = n_rows * sizeof(AttentionRow), block_bytes = table.size() * sizeof(unsigned);
+    char* memory = table_memory(ctx, n_rows, row_bytes + block_bytes, n_rows <= kInlineRows && blocks.size() <= kInlineBlocks);
+    if (memory == nullptr) {
+        std::memcpy(p.near_rows, rows, row_bytes);
+        std::memcpy(p.near_blocks, table.data(), block_bytes);
+    } else {
+        check(cudaMemcpyAsync(memory, rows, row_bytes, cudaMemcpyHostToDevice, stream), "cudaMemcpyAsync(rows)");
+        check(cudaMemcpyAsync(memory + row_bytes, table.data(), block_bytes, cudaMemcpyHostToDevice, stream), "cudaMemcpyAsync(table)");
+        p.far_rows = reinterpret_cast<const AttentionRow*>(memory);
+        p.far_blocks = reinterpret_cast<const unsigned*>(memory + row_bytes);
+    }
     p.heads = shape.heads;
     p.group = shape.heads / shape.kv_heads;
     p.scale_log2 = static_cast<float>(1.4426950408889634 / std::sqrt(static_cast<double>(D)));

@@ -104,6 +104,14 @@ def test_one_request_no_context(ctx, hd, rotary):
 
 
 @pytest.mark.parametrize("hd", [128, 256])
+def test_more_rows_than_travel_with_the_launch(ctx, hd):
+    """65 rows and more, or more than 160 blocks of queries, take their tables through device memory."""
+    run_case(ctx, heads=2, kv_heads=1, hd=hd, rotary=64, requests=[(3 * i % 7, 1 + i % 5) for i in range(65)], seed=9)
+    run_case(ctx, heads=2, kv_heads=1, hd=hd, rotary=64, requests=[(0, 12 + i % 3) for i in range(64)], seed=10)
+    run_case(ctx, heads=1, kv_heads=1, hd=hd, rotary=64, requests=[(0, 3)] + [(0, 520 + i) for i in range(59)], seed=11)  # 3 blocks of 256 each
+
+
+@pytest.mark.parametrize("hd", [128, 256])
 def test_context_and_several_requests(ctx, hd):
     run_case(ctx, heads=8, kv_heads=2, hd=hd, rotary=64, requests=[(0, 77), (200, 130), (513, 1), (64, 256), (1000, 300)], seed=7)
     run_case(ctx, heads=2, kv_heads=2, hd=hd, rotary=64, requests=[(4096, 512)], seed=8, in_half=False)
