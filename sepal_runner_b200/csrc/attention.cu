@@ -175,10 +175,66 @@ struct AttentionParams {
     const void* gate;
     unsigned long long gate_stride;
     unsigned gate_half;
+    unsigned gate_wide;  // binary16 rows that can be taken eight values at a time
     __half* out;
     unsigned long long out_stride;
     int* status;
 };
+
+// The last step of both kernels, a thread's N columns of its query: O / l * sigmoid(gate) from tensor memory to the output. A thread's
+// gates lie one after the other (and the warp's 32 rows apart), so they are fetched 16 bytes at a time, and before the last block's
+// products are waited for: value by value after them, this step was two thirds of a launch with few keys. All lanes take part in the loads
+// of tensor memory; only valid queries store.
+template <int N>
+__device__ __forceinline__ void fetch_gates(const AttentionParams& p, size_t gate0, bool live, uint4 (&gates)[N / 8]) {
+    if (p.gate_wide == 0 || !live) return;
+#pragma unroll
+    for (int i = 0; i < N / 8; ++i) gates[i] = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.gate) + gate0 + 8 * i);
+}
+
+__device__ __forceinline__ unsigned gated_pair(uint32_t o0, uint32_t o1, float inv_l, float g0, float g1) {
+    const __half2 h = __floats2half2_rn(__uint_as_float(o0) * inv_l * (1.0f / (1.0f + expf(-g0))), __uint_as_float(o1) * inv_l * (1.0f / (1.0f + expf(-g1))));
+    return *reinterpret_cast<const unsigned*>(&h);
+}
+
+template <int N>
+__device__ __forceinline__ void store_gated(const AttentionParams& p, uint32_t o_tmem, size_t gate0, const uint4 (&gates)[N / 8], __half* dst, bool live, float inv_l) {
+    if (p.gate_wide != 0) {
+#pragma unroll
+        for (int c = 0; c < N; c += 32) {
+            uint32_t v[32];
+            ptx::tmem_ld_32x32(o_tmem + c, v);
+            ptx::tmem_ld_wait();
+            if (!live) continue;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4 raw = gates[c / 8 + q];
+                const unsigned words[4] = {raw.x, raw.y, raw.z, raw.w};
+                unsigned packed[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 g = __half22float2(*reinterpret_cast<const __half2*>(&words[i]));
+                    packed[i] = gated_pair(v[8 * q + 2 * i], v[8 * q + 2 * i + 1], inv_l, g.x, g.y);
+                }
+                *reinterpret_cast<uint4*>(dst + c + 8 * q) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            }
+        }
+        return;
+    }
+#pragma unroll 1
+    for (int c = 0; c < N; c += 32) {
+        uint32_t v[32];
+        ptx::tmem_ld_32x32(o_tmem + c, v);
+        ptx::tmem_ld_wait();
+        if (!live) continue;
+        unsigned packed[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2)
+            packed[i / 2] = gated_pair(v[i], v[i + 1], inv_l, band_value(p.gate, gate0 + c + i, p.gate_half), band_value(p.gate, gate0 + c + i + 1, p.gate_half));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(dst + c + 8 * q) = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+    }
+}
 
 template <int D>
 struct AttentionTile {
@@ -424,38 +480,20 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             ptx::tc_fence_before_sync();
             ptx::mbar_arrive(p_full(s));
         }
+        const size_t token = static_cast<size_t>(row.q_begin) + q0 + r;
+        const size_t gate0 = token * p.gate_stride + static_cast<size_t>(head) * 2 * D + D + side * kDh;
+        uint4 gates[kDh / 8] = {};
+        fetch_gates<kDh>(p, gate0, r < valid, gates);
         if (ok && n_blocks > 0) ok = wait_barrier(p_free((n_blocks - 1) & 1u), ((n_blocks - 1) >> 1) & 1u, abort_flag, p.status, kStatusAttention + 7);
         // the row's sum: the first half's plus the second half's
         exchange[side * 128 + r] = l;
         pair_sync();
         const float total = exchange[r] + exchange[128 + r];
-        // every lane takes part in the loads; only valid queries store
         if (ok) {
             ptx::tc_fence_after_sync();
             const float inv_l = 1.0f / total;
-            const size_t token = static_cast<size_t>(row.q_begin) + q0 + r;
             __half* dst = p.out + token * p.out_stride + static_cast<size_t>(head) * D + side * kDh;
-            const size_t gate0 = token * p.gate_stride + static_cast<size_t>(head) * 2 * D + D + side * kDh;
-#pragma unroll 1
-            for (int c = 0; c < kDh; c += 32) {
-                uint32_t v[32];
-                ptx::tmem_ld_32x32(lane_base + T::kOCol + side * kDh + c, v);
-                ptx::tmem_ld_wait();
-                if (r < valid) {
-                    unsigned packed[16];
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float g0 = band_value(p.gate, gate0 + c + i, p.gate_half), g1 = band_value(p.gate, gate0 + c + i + 1, p.gate_half);
-                        const float o0 = __uint_as_float(v[i]) * inv_l * (1.0f / (1.0f + expf(-g0)));
-                        const float o1 = __uint_as_float(v[i + 1]) * inv_l * (1.0f / (1.0f + expf(-g1)));
-                        const __half2 h = __floats2half2_rn(o0, o1);
-                        packed[i / 2] = *reinterpret_cast<const unsigned*>(&h);
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        *reinterpret_cast<uint4*>(dst + c + 8 * q) = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-                }
-            }
+            store_gated<kDh>(p, lane_base + T::kOCol + side * kDh, gate0, gates, dst, r < valid, inv_l);
         }
     }
 
@@ -715,6 +753,10 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(p_full(sb), 0));  // one arrival for the warp
         }
+        const size_t token = static_cast<size_t>(row.q_begin) + q0 + r;
+        const size_t gate0 = token * p.gate_stride + static_cast<size_t>(head) * 2 * D + D + side * kDq;
+        uint4 gates[kDq / 8] = {};
+        fetch_gates<kDq>(p, gate0, r < valid, gates);
         if (ok && n_blocks > 0) {
             const unsigned last = n_blocks - 1;
             ok = wait_barrier(p_free(last & 1u), (last >> 1) & 1u, abort_flag, p.status, kStatusAttention + 7);
@@ -725,29 +767,8 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (ok) {
             ptx::tc_fence_after_sync();
             const float inv_l = 1.0f / total;
-            const size_t token = static_cast<size_t>(row.q_begin) + q0 + r;
             __half* dst = p.out + token * p.out_stride + static_cast<size_t>(head) * D + side * kDq;
-            const size_t gate0 = token * p.gate_stride + static_cast<size_t>(head) * 2 * D + D + side * kDq;
-#pragma unroll 1
-            for (int c = 0; c < kDq; c += 32) {
-                uint32_t v[32];
-                ptx::tmem_ld_32x32(lane_base + T::kOCol + side * kDq + c, v);
-                ptx::tmem_ld_wait();
-                if (r < valid) {
-                    unsigned packed[16];
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float g0 = band_value(p.gate, gate0 + c + i, p.gate_half), g1 = band_value(p.gate, gate0 + c + i + 1, p.gate_half);
-                        const float o0 = __uint_as_float(v[i]) * inv_l * (1.0f / (1.0f + expf(-g0)));
-                        const float o1 = __uint_as_float(v[i + 1]) * inv_l * (1.0f / (1.0f + expf(-g1)));
-                        const __half2 h = __floats2half2_rn(o0, o1);
-                        packed[i / 2] = *reinterpret_cast<const unsigned*>(&h);
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        *reinterpret_cast<uint4*>(dst + c + 8 * q) = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-                }
-            }
+            store_gated<kDq>(p, lane_base + T::kOCol + side * kDq, gate0, gates, dst, r < valid, inv_l);
         }
     }
 
@@ -886,6 +907,7 @@ void launch_attention(Context& ctx, const AttentionShape& shape, const Attention
     p.gate = gate.data;
     p.gate_stride = gate.stride;
     p.gate_half = gate.half ? 1u : 0u;
+    p.gate_wide = gate.half && gate.stride % 8 == 0 && reinterpret_cast<std::uintptr_t>(gate.data) % 16 == 0 ? 1u : 0u;
     p.out = static_cast<__half*>(out);
     p.out_stride = out_stride;
     p.status = ctx.status;
