@@ -151,6 +151,10 @@ __device__ __forceinline__ float4 input_pairs_before(const DeltaParams& p, const
 // A warp takes 128 channels (a head of q or k, or 128 channels of v) of eight consecutive tokens, lane l the channels 2 l, 2 l + 1,
 // 64 + 2 l and 65 + 2 l: eleven rows are read for eight tokens, all in flight at once, and the taps once. `Pairs`: binary16 inputs and
 // four taps at addresses that allow two channels a load; otherwise channel by channel.
+//
+// What bounds it is instructions (61 % of the issue slots, the shared-memory pipe at 41 %): five runs of 2500 tokens in all, 32 value
+// heads, 69 us, where the convolution and the coefficients as two launches, with q and k written and read back between them, took
+// 74 + 65 us under the profiler. Four blocks to an SM hide one another's barriers (4096 tokens: 98 us, 104 with three).
 constexpr int kHeadsAtOnce = 2;
 
 template <bool Pairs>
@@ -406,6 +410,11 @@ __device__ __forceinline__ void add_to(float4& sum, const float4& v) { sum.x += 
 // global memory as they do here: many small ones take longer to issue than the chunk's arithmetic; cp.async for the block's columns of
 // v). The reads go to global memory in float32; the gated norm over a head's 128 reads is the next launch.
 //
+// One run, 32 value heads: 0.86 us a chunk, 54 ns a token (with one warp to sixteen columns 82 ns), and that is the latency of the chain:
+// the same without any copies, issue slots 38 %, tensor pipe 20 %, shared-memory pipe 41 %. Parts 2 and sixteen columns to a warp were
+// the best of ten layouts (900 tokens: 53 us; four parts 63; one set of two by two 66; 64 columns to a block 78). Fetching the last
+// product's operands in the middle of the first products gave 9 %; 16-byte loads of k and q (fewer instructions) lost 5 %.
+//
 // Tokens within a tile of eight: column j of an accumulator tile is token (0, 2, 1, 3, 6, 4, 7, 5)[j]. With that order both ways k is
 // read (eight tokens' pairs of dimensions as the B operand of the first products, four pairs of tokens as that of the last) touch every
 // bank once.
@@ -636,17 +645,23 @@ void launch_scan(const Context& ctx, const DeltaParams& p, cudaStream_t stream) 
         check(cudaFuncSetAttribute(deltanet_scan_kernel<Parts, Wide, Sets>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(typename Shape::Smem))), "cudaFuncSetAttribute");
         if (ctx.device < 64) configured[ctx.device].store(true, std::memory_order_relaxed);
     }
-    // An ordinary launch, not an overlapped one: blocks of the scan that arrive while the launch before it still fills the SMs settle
-    // wherever room appears first, several to an SM with other SMs left empty, and a run's warps then take twice as long.
-    deltanet_scan_kernel<Parts, Wide, Sets><<<dim3(p.n_rows * p.value_heads * (kDim / Shape::kColumns)), dim3(Shape::kThreads), sizeof(typename Shape::Smem), stream>>>(p);
-    check(cudaGetLastError(), "deltanet_scan_kernel launch");
+    // Overlapped with the launch before it only where that has a block to an SM at most: blocks of the scan that arrive while it still fills
+    // the SMs settle wherever room appears first, several to an SM with other SMs left empty, and a run's warps then take twice as long.
+    const dim3 grid(p.n_rows * p.value_heads * (kDim / Shape::kColumns)), block(Shape::kThreads);
+    if (p.n_chunks * p.key_heads <= static_cast<unsigned>(ctx.sm_count)) {
+        launch_kernel(deltanet_scan_kernel<Parts, Wide, Sets>, grid, block, sizeof(typename Shape::Smem), stream, "deltanet_scan_kernel launch", p);
+    } else {
+        deltanet_scan_kernel<Parts, Wide, Sets><<<grid, block, sizeof(typename Shape::Smem), stream>>>(p);
+        check(cudaGetLastError(), "deltanet_scan_kernel launch");
+    }
     count_launch();
 }
 
 // The gated norm of every token's and value head's 128 reads: x / sqrt(mean(x^2) + eps) * weight * silu(z) (the weight itself, not
 // 1 + weight). A warp takes four (token, head) pairs in a row, all their loads in flight together; lane l holds reads 4 l to 4 l + 3;
 // squares by fused multiply-add in that order, a butterfly. The last blocks leave the slots' tails as the last K - 1 rows of (old tail,
-// then the run's inputs): the launch that read the old ones is complete.
+// then the run's inputs): the launch that read the old ones is complete. 4096 tokens, 32 heads, 134 MB: 45 us, bound by instructions
+// (53 with the divisions of a 64-bit unit number).
 constexpr unsigned kNormUnits = 4;
 
 __global__ void __launch_bounds__(256) deltanet_norm_kernel(const __grid_constant__ DeltaParams p, unsigned norm_blocks) {

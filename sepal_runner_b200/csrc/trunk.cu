@@ -66,7 +66,8 @@ __global__ void embed_kernel(const __half* table, const std::uint32_t* tokens, f
 //
 // A block of 256 threads owns a row, thread i the partial sum number i. What bounds the launch between two multiplies is the latency of
 // a row, not its bytes (which the L2 still holds), so a thread has at most kNormHeld chunks, their loads and the gains' in flight at
-// once, and the row meets at one barrier. Rows wider than the registers hold are read a second time.
+// once, and the row meets at one barrier. (A warp to a row, with 80 divisions to a lane: 8.8 us for 29 rows of 1024 under the profiler.)
+// Rows wider than the registers hold are read a second time.
 constexpr unsigned kNormThreads = 256;
 constexpr int kNormHeld = 4;  // chunks a thread keeps: rows up to 4096 wide
 
