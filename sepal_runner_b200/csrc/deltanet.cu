@@ -62,10 +62,10 @@ __device__ __forceinline__ float value_of(const void* base, unsigned long long i
     return half != 0 ? __half2float(static_cast<const __half*>(base)[index]) : static_cast<const float*>(base)[index];
 }
 // softplus in the reference's form (runner/include/sepal/ref/primitives.hpp:25-40); sigmoid as 1 / (1 + e^-x), which the reference
-// writes as exp(-softplus(-x)): the same function, an ulp or two apart in float32, and a fifth of the instructions (it runs once per
-// element of the convolution's output and of the gate, and the kernels that do are bound by their instructions).
+// writes as exp(-softplus(-x)): the same function, an ulp or two apart in float32, and a third of the instructions (it runs once per
+// element of the convolution's output and of the gate). The quotient is rounded to nearest: beta and the activated k enter a recurrence.
 __device__ __forceinline__ float softplus(float x) { return fmaxf(x, 0.0f) + log1pf(expf(-fabsf(x))); }
-__device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.0f, __fadd_rn(1.0f, expf(-x))); }
+__device__ __forceinline__ float sigmoid(float x) { return __frcp_rn(__fadd_rn(1.0f, expf(-x))); }
 __device__ __forceinline__ float silu(float x) { return __fmul_rn(x, sigmoid(x)); }
 
 __device__ __forceinline__ uint32_t to_tf32(float x) {

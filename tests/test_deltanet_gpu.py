@@ -154,6 +154,62 @@ def test_layouts_agree(ctx, value_heads, runs, length):
     assert (got[0][0][~live.cuda()] == 7.0).all()
 
 
+def one_token_runs(ctx, key_heads, value_heads, runs, q, k, v, z, norm):
+    """Fresh runs of one token each: the convolution hands q, k and v (float32 [runs, width]) through, beta is exactly 1. Returns the
+    output [runs, value_heads, 128] and the states [runs, value_heads, 128, 128]. With no state before the token the chunk's products
+    are single products: S = k (x) v and read = (q . k) v / sqrt(128), the operands rounded to TF32."""
+    import torch
+
+    import sepal_runner_b200 as sb
+
+    dim = 128
+    shape = sb.DeltaNetShape(key_heads=key_heads, value_heads=value_heads, head_dim=dim, conv_kernel=4, eps=1e-6)
+    vd, cd = value_heads * dim, (2 * key_heads + value_heads) * dim
+    taps = torch.zeros((cd, 4), device="cuda")
+    taps[:, 3] = 1.0
+    gate = torch.full((runs, value_heads), 100.0, device="cuda")  # 1 + e^-100 is 1
+    states = torch.empty((runs, value_heads, dim, dim), device="cuda")
+    tails = torch.empty((runs, 3, cd), device="cuda")
+    out = torch.empty((runs, vd), dtype=torch.float16, device="cuda")
+    zero = torch.zeros(value_heads, device="cuda")
+    keep = sb.deltanet(ctx, shape, [(i, 1, i, 1) for i in range(runs)], torch.cat([q, k, v], dim=1), z, gate, torch.zeros_like(gate), taps, zero, zero, norm,
+                       states, tails, out)
+    ctx.check_status()
+    del keep
+    return out.view(runs, value_heads, dim), states
+
+
+def tf32(x):
+    """float32 rounded to TF32 (10 bits of mantissa), to nearest, ties away from zero, as cvt.rna does."""
+    import torch
+
+    return ((x.view(torch.int32) + 0x1000) & ~0x1FFF).view(torch.float32)
+
+
+def one_hot(runs, heads):
+    """1000 in dimension 0 of every head: silu(1000) is 1000 and its l2-normalised head exactly (1, 0, 0, ...)."""
+    import torch
+
+    x = torch.zeros((runs, heads, 128), device="cuda")
+    x[:, :, 0] = 1000.0
+    return x.view(runs, heads * 128)
+
+
+def test_silu_divides_to_nearest(ctx):
+    """silu(x) = x * (1 / (1 + e^-x)) with every operation rounded to nearest, 410 thousand values: a quotient an ulp off shows where it
+    crosses one of the 8192 ulps between two TF32 numbers."""
+    import torch
+
+    runs, key_heads, value_heads = 200, 2, 16
+    gen = torch.Generator(device="cuda").manual_seed(21)
+    v = torch.randn((runs, value_heads * 128), generator=gen, device="cuda") * 3
+    hot = one_hot(runs, key_heads)
+    _, states = one_token_runs(ctx, key_heads, value_heads, runs, hot, hot, v, torch.zeros_like(v), torch.ones(128, device="cuda"))
+    want = tf32(v * (1.0 / (1.0 + torch.exp(-v))))
+    assert torch.equal(states[:, :, 0, :].reshape(runs, -1), want)
+    assert (states[:, :, 1:, :] == 0).all()
+
+
 def test_arguments_are_checked(ctx):
     import torch
 
