@@ -245,9 +245,9 @@ __global__ void __launch_bounds__(256, 4) deltanet_prepare_kernel(const __grid_c
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const bool live = first + i < count;
-            const float unit = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(ss[i], 1.0e-6f)));
-            const float n[4] = {live ? __fmul_rn(act[i].x, unit) : 0.0f, live ? __fmul_rn(act[i].y, unit) : 0.0f, live ? __fmul_rn(act[i].z, unit) : 0.0f,
-                                live ? __fmul_rn(act[i].w, unit) : 0.0f};
+            const float norm = __fsqrt_rn(__fadd_rn(ss[i], 1.0e-6f));  // (a division, not a multiplication by 1 / norm, which would round twice)
+            const float n[4] = {live ? __fdiv_rn(act[i].x, norm) : 0.0f, live ? __fdiv_rn(act[i].y, norm) : 0.0f, live ? __fdiv_rn(act[i].z, norm) : 0.0f,
+                                live ? __fdiv_rn(act[i].w, norm) : 0.0f};
             float* row = (part == 0 ? q_sh : k_sh)[first + i] + 2 * lane;
             *reinterpret_cast<float2*>(row) = make_float2(n[0], n[1]);
             *reinterpret_cast<float2*>(row + 64) = make_float2(n[2], n[3]);

@@ -210,6 +210,23 @@ def test_silu_divides_to_nearest(ctx):
     assert (states[:, :, 1:, :] == 0).all()
 
 
+def test_heads_are_normalised_by_one_division(ctx):
+    """k / sqrt(sum k^2 + 1e-6), rounded once: whole numbers from 20 up pass the SiLU unchanged and their squares add up exactly, so numpy's
+    float32 says what every one of the 410 thousand quotients is."""
+    import torch
+
+    runs, heads = 200, 16
+    rng = np.random.default_rng(22)
+    k = rng.integers(20, 300, (runs, heads, 128)).astype(np.float32)
+    norm = np.sqrt((k * k).sum(-1, dtype=np.float32, keepdims=True) + np.float32(1e-6))
+    assert (k.astype(np.int64) ** 2).sum(-1).max() < 1 << 24
+    kd = torch.from_numpy(k).cuda().view(runs, heads * 128)
+    v = torch.full((runs, heads * 128), 32.0, device="cuda")
+    _, states = one_token_runs(ctx, heads, heads, runs, kd, kd, v, torch.zeros_like(v), torch.ones(128, device="cuda"))
+    want = tf32(torch.from_numpy(k / norm).cuda()) * 32.0
+    assert torch.equal(states, want[:, :, :, None].expand_as(states))
+
+
 def test_arguments_are_checked(ctx):
     import torch
 
