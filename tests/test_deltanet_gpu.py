@@ -227,6 +227,31 @@ def test_heads_are_normalised_by_one_division(ctx):
     assert torch.equal(states, want[:, :, :, None].expand_as(states))
 
 
+def test_gated_norm_divides_once(ctx):
+    """(read / rms) * weight * silu(z) with each of the three operations rounded once. Reads are whole numbers times 1 / sqrt(128), their
+    squares summed by fused multiply-adds over four neighbours and then by halves of the warp; silu(32) is 32."""
+    import torch
+
+    runs, heads = 200, 16
+    rng = np.random.default_rng(23)
+    v = rng.integers(20, 2000, (runs, heads, 128)).astype(np.float32)
+    weight = (1.0 + 0.1 * rng.standard_normal(128)).astype(np.float32)
+    hot = one_hot(runs, heads)
+    vd = torch.from_numpy(v).cuda().view(runs, heads * 128)
+    out, _ = one_token_runs(ctx, heads, heads, runs, hot, hot, vd, torch.full_like(vd, 32.0), torch.from_numpy(weight).cuda())
+    x = v * np.float32(128 ** -0.5)
+    lane = x.reshape(runs, heads, 32, 4)
+    ss = np.zeros(lane.shape[:3], np.float32)
+    for e in range(4):
+        ss = (lane[..., e].astype(np.float64) ** 2 + ss).astype(np.float32)
+    while ss.shape[-1] > 1:
+        half = ss.shape[-1] // 2
+        ss = ss[..., :half] + ss[..., half:]
+    rms = np.sqrt(ss / np.float32(128) + np.float32(1e-6))
+    want = ((x / rms) * weight * np.float32(32)).astype(np.float16)
+    assert np.array_equal(out.cpu().numpy(), want)
+
+
 def test_arguments_are_checked(ctx):
     import torch
 
