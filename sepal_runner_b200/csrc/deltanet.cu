@@ -403,10 +403,26 @@ __device__ __forceinline__ bool scan_wait(uint32_t bar, uint32_t parity, unsigne
 
 __device__ __forceinline__ void add_to(float4& sum, const float4& v) { sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w; }
 
+// The slot's tail becomes the last K - 1 rows of (old tail, then the run's inputs): one warp's share of the channels, `part` of `parts`.
+// In the scan, because the launch before it has read the old tail by then and the launch after it may write over the inputs (`out` may lie
+// on `mixed`).
+__device__ __forceinline__ void leave_tail(const DeltaParams& p, const DeltaNetRow& run, unsigned part, unsigned parts, unsigned lane) {
+    const unsigned history = p.taps - 1, share = (p.conv_dim + parts - 1) / parts;
+    float* tail = p.tails + static_cast<size_t>(run.slot) * history * p.conv_dim;
+    for (unsigned c = part * share + lane; c < min((part + 1) * share, p.conv_dim); c += 32) {
+        float x[7];  // all rows before the first is written: a run shorter than the tail moves its old rows up
+#pragma unroll
+        for (unsigned i = 0; i < 7; ++i) x[i] = i < history ? input_at(p, run, tail, static_cast<int>(run.length + i) - static_cast<int>(history), c) : 0.0f;
+#pragma unroll
+        for (unsigned i = 0; i < 7; ++i)
+            if (i < history) tail[static_cast<size_t>(i) * p.conv_dim + c] = x[i];
+    }
+}
+
 // One block per run, value head and ScanShape::kColumns columns of the state (columns evolve independently of one another). A chunk's
 // chain is state -> products with it -> y -> T2 y -> state. The warps of a set hold their part of the state in registers and exchange
 // partial sums through shared memory once a chunk (each then forms y and T2 y for itself). What hangs off the chain is not theirs: one
-// more warp a set adds up the reads, a last one brings the chunks (two bulk copies a chunk for k, q and the coefficients, which lie in
+// more warp a set adds up the reads, a last one brings the chunks and then leaves the tail (two bulk copies a chunk for k, q and the coefficients, which lie in
 // global memory as they do here: many small ones take longer to issue than the chunk's arithmetic; cp.async for the block's columns of
 // v). The reads go to global memory in float32; the gated norm over a head's 128 reads is the next launch.
 //
@@ -474,6 +490,7 @@ __global__ void __launch_bounds__(ScanShape<Parts, Wide, Sets>::kThreads) deltan
             }
             ptx::cp_async_mbar_arrive(bar);
         }
+        leave_tail(p, row, head * (kDim / Shape::kColumns) + columns, p.value_heads * (kDim / Shape::kColumns), lane);
         ptx::grid_launch_dependents();
         return;
     }
@@ -665,25 +682,13 @@ void launch_scan(const Context& ctx, const DeltaParams& p, cudaStream_t stream) 
 
 // The gated norm of every token's and value head's 128 reads: x / sqrt(mean(x^2) + eps) * weight * silu(z) (the weight itself, not
 // 1 + weight). A warp takes four (token, head) pairs in a row, all their loads in flight together; lane l holds reads 4 l to 4 l + 3;
-// squares by fused multiply-add in that order, a butterfly. The last blocks leave the slots' tails as the last K - 1 rows of (old tail,
-// then the run's inputs): the launch that read the old ones is complete. 4096 tokens, 32 heads, 134 MB: 45 us, bound by instructions
-// (53 with the divisions of a 64-bit unit number).
+// squares by fused multiply-add in that order, a butterfly. 4096 tokens, 32 heads, 134 MB: 45 us, bound by instructions (53 with the
+// divisions of a 64-bit unit number).
 constexpr unsigned kNormUnits = 4;
 
-__global__ void __launch_bounds__(256) deltanet_norm_kernel(const __grid_constant__ DeltaParams p, unsigned norm_blocks) {
+__global__ void __launch_bounds__(256) deltanet_norm_kernel(const __grid_constant__ DeltaParams p) {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
-    if (blockIdx.x >= norm_blocks) {
-        const unsigned per_run = (p.conv_dim + 255) / 256, at = blockIdx.x - norm_blocks;
-        const DeltaNetRow run = run_at(p, at / per_run);
-        const unsigned history = p.taps - 1, c = at % per_run * 256 + threadIdx.x;
-        float* tail = p.tails + static_cast<size_t>(run.slot) * history * p.conv_dim;
-        if (c < p.conv_dim) {
-            for (unsigned i = 0; i < history; ++i)  // ascending: row length + i of the window is read before row i is written (length >= 1)
-                tail[static_cast<size_t>(i) * p.conv_dim + c] = input_at(p, run, tail, static_cast<int>(run.length + i) - static_cast<int>(history), c);
-        }
-        return;
-    }
     const unsigned lane = threadIdx.x % 32;
     const unsigned first = (blockIdx.x * 8 + threadIdx.x / 32) * kNormUnits, units = p.n_tokens * p.value_heads;
     const float4 weight = make_float4(p.norm[4 * lane], p.norm[4 * lane + 1], p.norm[4 * lane + 2], p.norm[4 * lane + 3]);
@@ -830,9 +835,8 @@ void launch_deltanet(Context& ctx, const DeltaNetShape& shape, const DeltaNetRow
     else
         launch_scan<2, 1, 2>(ctx, p, stream);
     const std::size_t units = static_cast<std::size_t>(last) * shape.value_heads;
-    const unsigned norm_blocks = static_cast<unsigned>((units + 8 * kNormUnits - 1) / (8 * kNormUnits));
-    const unsigned tail_blocks = shape.conv_kernel > 1 ? p.n_rows * ((p.conv_dim + 255) / 256) : 0u;
-    launch_kernel(deltanet_norm_kernel, dim3(norm_blocks + tail_blocks), dim3(256), 0, stream, "deltanet_norm_kernel launch", p, norm_blocks);
+    launch_kernel(deltanet_norm_kernel, dim3(static_cast<unsigned>((units + 8 * kNormUnits - 1) / (8 * kNormUnits))), dim3(256), 0, stream,
+                  "deltanet_norm_kernel launch", p);
     count_launch();
 }
 

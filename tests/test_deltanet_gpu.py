@@ -252,6 +252,33 @@ def test_gated_norm_divides_once(ctx):
     assert np.array_equal(out.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("value_heads,lengths,taps", [(4, (1, 2, 3, 40), 4), (16, (130, 17), 4), (8, (1, 3, 5, 20), 8), (2, tuple(1 + 2 * (i % 9) for i in range(70)), 4)])
+def test_output_on_the_inputs(ctx, value_heads, lengths, taps):
+    """`out` on the first columns of `mixed`: the inputs have been read, those of the tails included, before the output overwrites them."""
+    import torch
+
+    import sepal_runner_b200 as sb
+
+    key_heads, dim = 2, 128
+    shape = sb.DeltaNetShape(key_heads=key_heads, value_heads=value_heads, head_dim=dim, conv_kernel=taps, eps=1e-6)
+    vd, cd = value_heads * dim, (2 * key_heads + value_heads) * dim
+    gen = torch.Generator(device="cuda").manual_seed(value_heads)
+    normal = lambda *s: torch.randn(s, generator=gen, device="cuda")  # noqa: E731
+    rows = [(sum(lengths[:i]), n, i, i % 2) for i, n in enumerate(lengths)]
+    conv, a_log, dt_bias, norm = normal(cd, taps) * 0.5, normal(value_heads), normal(value_heads), 1 + normal(dim) * 0.1
+    states, tails = normal(len(rows), value_heads, dim, dim) * 0.05, normal(len(rows), taps - 1, cd)
+    mixed, z, b, a = [normal(sum(lengths), w).half() for w in (cd, vd, value_heads, value_heads)]
+    got = []
+    for out in (torch.empty((sum(lengths), vd), dtype=torch.float16, device="cuda"), mixed[:, :vd]):
+        st, tl = states.clone(), tails.clone()
+        keep = sb.deltanet(ctx, shape, rows, mixed, z, b, a, conv, a_log, dt_bias, norm, st, tl, out)
+        ctx.check_status()
+        del keep
+        got.append((out.clone(), st, tl))
+    for x, y in zip(*got):
+        assert torch.isfinite(x).all() and torch.equal(x, y)
+
+
 def test_arguments_are_checked(ctx):
     import torch
 
