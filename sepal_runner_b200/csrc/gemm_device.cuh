@@ -33,6 +33,13 @@ __device__ __forceinline__ bool wait_barrier(uint32_t bar, uint32_t parity, vola
     }
 }
 
+// Barriers of a ring of `depth` slots whose uses two waiters take in turn (use i: slot i % depth, waiter i % 2, barrier i % this). A wait
+// names a phase by its parity and is only right when the waiter has seen the phase before it. With an odd depth and a barrier to a
+// slot, a barrier's phases would go to the two waiters alternately: one that has run ahead (loads may land out of order) then asks for
+// the next phase while the other's is still open, and passes at once on the parity of the phase before that. An even number of barriers
+// gives each of them to one waiter.
+__host__ __device__ constexpr unsigned barriers_in_turn(unsigned depth) { return depth % 2 != 0 ? 2 * depth : depth; }
+
 // A producer that gives up in a pair kernel cannot wait on barriers for the copies it still has in flight (some complete on the other
 // CTA's barriers): it gives them a bounded time to land, many times what a TMA load takes, before its CTA may release shared memory.
 __device__ __forceinline__ void grace_for_copies_in_flight() {

@@ -90,7 +90,8 @@ constexpr int kMaxStages = 8;
 constexpr int kXBytes = kBM * kBK * 2;              // one X tile: 128 rows of 128 bytes
 constexpr int kAccStride = 256;                     // tensor-memory columns between the two accumulators
 constexpr int kTmemCols = 512;
-constexpr int kBarriers = 2 * kMaxStages + 4 + 4 + 2;   // full, empty, accumulator full / empty, converted full / empty, fix-up
+constexpr int kFullBars = 2 * kMaxStages;           // (see barriers_in_turn)
+constexpr int kBarriers = kFullBars + kMaxStages + 4 + 4 + 2;   // full, empty, accumulator full / empty, converted full / empty, fix-up
 constexpr int kTailBytes = kBarriers * 8 + 64;
 constexpr int kSmemLimit = 232448;                  // 227 KB: the most one CTA may have
 constexpr int kStagingBox = kBM * 128;              // one [128 rows x 32 float32] box of the staged residual epilogue
@@ -811,11 +812,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     uint8_t* const tail = smem + stages * stage_bytes + S::kConvBuffers * conv_bytes;
     const uint32_t bars = ptx::smem_addr(tail);
     const auto full_bar = [&](int s) { return bars + 8u * s; };
-    const auto empty_bar = [&](int s) { return bars + 8u * (kMaxStages + s); };
-    const auto acc_full_bar = [&](int a) { return bars + 8u * (2 * kMaxStages + a); };
-    const auto acc_empty_bar = [&](int a) { return bars + 8u * (2 * kMaxStages + 2 + a); };
-    const auto conv_full_bar = [&](int c) { return bars + 8u * (2 * kMaxStages + 4 + c); };
-    const auto conv_empty_bar = [&](int c) { return bars + 8u * (2 * kMaxStages + 6 + c); };
+    const auto empty_bar = [&](int s) { return bars + 8u * (kFullBars + s); };
+    const auto acc_full_bar = [&](int a) { return bars + 8u * (kFullBars + kMaxStages + a); };
+    const auto acc_empty_bar = [&](int a) { return bars + 8u * (kFullBars + kMaxStages + 2 + a); };
+    const auto conv_full_bar = [&](int c) { return bars + 8u * (kFullBars + kMaxStages + 4 + c); };
+    const auto conv_empty_bar = [&](int c) { return bars + 8u * (kFullBars + kMaxStages + 6 + c); };
+    const unsigned fulls = p.issuers == 2 ? barriers_in_turn(p.stages) : p.stages;  // step i arrives on barrier i % fulls
     unsigned* const words = reinterpret_cast<unsigned*>(tail + kBarriers * 8);
     unsigned* const tmem_slot = words;                 // base address of the tensor memory allocation
     volatile unsigned* const abort_flag = words + 1;   // raised by the first wait that runs out
@@ -825,10 +827,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     const unsigned grid = gridDim.x, cta = blockIdx.x;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; ++s) {
-            ptx::mbar_init(full_bar(s), 1);
-            ptx::mbar_init(empty_bar(s), W8 ? 1 + 4 : 1);  // the MMA's commit (+ one arrival per converter warp)
-        }
+        for (unsigned s = 0; s < fulls; ++s) ptx::mbar_init(full_bar(s), 1);
+        for (int s = 0; s < stages; ++s) ptx::mbar_init(empty_bar(s), W8 ? 1 + 4 : 1);  // the MMA's commit (+ one arrival per converter warp)
         for (int a = 0; a < 2; ++a) {
             ptx::mbar_init(acc_full_bar(a), a == 0 ? p.issuers : 1u);  // two issuing threads share the first accumulator's hand-over
             ptx::mbar_init(acc_empty_bar(a), 128);
@@ -885,9 +885,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         ptx::tc_fence_after_sync();
         const uint32_t d = tmem_base + turn * kAccStride;
         int stage = static_cast<int>(turn);  // the ring holds at least two stages
-        unsigned phase = 0, fresh = 0;
+        unsigned full = turn, phase = 0, fresh = 0;
         for (unsigned kk = kb + turn; kk < ke; kk += 2) {
-            if (!wait_barrier(full_bar(stage), phase, abort_flag, p.status, kStatusMmaFull)) return;
+            if (!wait_barrier(full_bar(full), phase, abort_flag, p.status, kStatusMmaFull)) return;
             ptx::tc_fence_after_sync();
             const uint64_t step = static_cast<uint64_t>(static_cast<uint32_t>(stage) * stage_step);
             ptx::mma_f16_ss(d, desc_x0 + step, desc_w0 + step, idesc, fresh);  // this thread's first MMA overwrites its accumulator
@@ -896,8 +896,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             for (int j = 1; j < kBK / 16; ++j) ptx::mma_f16_ss(d, desc_x0 + step + 2u * j, desc_w0 + step + 2u * j, idesc, 1u);
             ptx::mma_commit(empty_bar(stage));
             stage += 2;
-            if (stage >= stages) {
-                stage -= stages;
+            if (stage >= stages) stage -= stages;
+            full += 2;
+            if (full == fulls + turn) {  // (fulls is even)
+                full = turn;
                 phase ^= 1u;
             }
         }
@@ -911,7 +913,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             unsigned tile, kb, ke;
             int stage = 0;
             unsigned phase = 0;
-            unsigned issued = 0;  // stages filled so far (for the drain below)
+            unsigned issued = 0, full = 0;  // stages filled so far (for the drain below); the barrier of the next
             bool ok = true;
             while (ok && walk.next(tile, kb, ke)) {
                 const unsigned m_tile = tile % p.m_tiles, n_tile = tile / p.m_tiles;
@@ -922,10 +924,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                         break;
                     }
                     const uint32_t dst = stages_addr + stage * stage_bytes;
-                    if (!begun) ptx::mbar_arrive_expect_tx(full_bar(stage), stage_bytes);
-                    ptx::tma_load_2d(dst, &map_x, full_bar(stage), static_cast<int>(kk * kBK), static_cast<int>(m_tile * kBM));
-                    if (!begun) ptx::tma_load_2d(dst + kXBytes, &map_w, full_bar(stage), static_cast<int>(kk * kBK), static_cast<int>(n_tile * bn));
+                    if (!begun) ptx::mbar_arrive_expect_tx(full_bar(full), stage_bytes);
+                    ptx::tma_load_2d(dst, &map_x, full_bar(full), static_cast<int>(kk * kBK), static_cast<int>(m_tile * kBM));
+                    if (!begun) ptx::tma_load_2d(dst + kXBytes, &map_w, full_bar(full), static_cast<int>(kk * kBK), static_cast<int>(n_tile * bn));
                     ++issued;
+                    if (++full == fulls) full = 0;
                     if (++stage == stages) {
                         stage = 0;
                         phase ^= 1u;
@@ -935,16 +938,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             if (!ok) {
                 // Giving up: let the copies still in flight land before the CTA's shared memory is released. The last
                 // min(issued, stages) fills are the ones that may not have been consumed; each has its own full barrier.
-                const unsigned pending = issued < static_cast<unsigned>(stages) ? issued : static_cast<unsigned>(stages);
-                int s = stage;
-                unsigned ph = phase;
-                for (unsigned i = 0; i < pending; ++i) {
-                    if (--s < 0) {
-                        s = stages - 1;
-                        ph ^= 1u;
-                    }
+                for (unsigned i = issued < p.stages ? 0u : issued - p.stages; i < issued; ++i) {
                     const long long t0 = clock64();
-                    while (!ptx::mbar_try_wait(full_bar(s), ph) && clock64() - t0 < (1ll << 24)) {
+                    while (!ptx::mbar_try_wait(full_bar(i % fulls), (i / fulls) & 1u) && clock64() - t0 < (1ll << 24)) {
                     }
                 }
             }
@@ -1158,9 +1154,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     uint8_t* const tail = smem + stages * stage_bytes;
     const uint32_t bars = ptx::smem_addr(tail);
     const auto full_bar = [&](int s) { return bars + 8u * s; };
-    const auto empty_bar = [&](int s) { return bars + 8u * (kMaxStages + s); };
-    const auto acc_full_bar = [&](int a) { return bars + 8u * (2 * kMaxStages + a); };
-    const auto acc_empty_bar = [&](int a) { return bars + 8u * (2 * kMaxStages + 2 + a); };
+    const auto empty_bar = [&](int s) { return bars + 8u * (kFullBars + s); };
+    const auto acc_full_bar = [&](int a) { return bars + 8u * (kFullBars + kMaxStages + a); };
+    const auto acc_empty_bar = [&](int a) { return bars + 8u * (kFullBars + kMaxStages + 2 + a); };
     unsigned* const words = reinterpret_cast<unsigned*>(tail + kBarriers * 8);
     unsigned* const tmem_slot = words;
     volatile unsigned* const abort_flag = words + 1;
