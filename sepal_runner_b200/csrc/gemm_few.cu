@@ -41,7 +41,9 @@ constexpr unsigned kThreads = 320;
 constexpr unsigned kMaxStages = 8;
 constexpr unsigned kMaxABufs = 4;
 constexpr unsigned kWBytes = kRows * 128;   // one box of W: 64 binary16 or 128 int8 values of k
-constexpr unsigned kTailBytes = (2 * kMaxStages + 2 * kMaxABufs + 1) * 8 + 64;
+constexpr unsigned kFullBars = 2 * kMaxStages;  // (see barriers_in_turn)
+constexpr unsigned kBarriers = kFullBars + kMaxStages + 2 * kMaxABufs + 1;
+constexpr unsigned kTailBytes = kBarriers * 8 + 64;
 constexpr unsigned kSmemMax = 232448;
 constexpr unsigned kSmemHalf = 112 * 1024;  // two CTAs to an SM, with what the system takes of its 228 KB
 
@@ -119,11 +121,15 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     uint8_t* const tail = smem + scale_off + (W8 ? p.stages * 256 : 0);
     const uint32_t bars = ptx::smem_addr(tail);
     const auto full_bar = [&](int s) { return bars + 8u * s; };
-    const auto empty_bar = [&](int s) { return bars + 8u * (kMaxStages + s); };
-    const auto a_full_bar = [&](int s) { return bars + 8u * (2 * kMaxStages + s); };
-    const auto a_empty_bar = [&](int s) { return bars + 8u * (2 * kMaxStages + kMaxABufs + s); };
-    const uint32_t acc_bar = bars + 8u * (2 * kMaxStages + 2 * kMaxABufs);
-    unsigned* const words = reinterpret_cast<unsigned*>(tail + (2 * kMaxStages + 2 * kMaxABufs + 1) * 8);
+    const auto empty_bar = [&](int s) { return bars + 8u * (kFullBars + s); };
+    const auto a_full_bar = [&](int s) { return bars + 8u * (kFullBars + kMaxStages + s); };
+    const auto a_empty_bar = [&](int s) { return bars + 8u * (kFullBars + kMaxStages + kMaxABufs + s); };
+    const uint32_t acc_bar = bars + 8u * (kBarriers - 1);
+    unsigned* const words = reinterpret_cast<unsigned*>(tail + kBarriers * 8);
+    // Step i arrives on full barrier i % fulls: the two sets of converters take the ring's slots in turn. (What they wait for before they
+    // reuse a weight buffer, the one issuing thread's commits, completes in order: a set that has seen the commit two steps back has seen
+    // every phase before.)
+    const int fulls = static_cast<int>(W8 ? barriers_in_turn(p.stages) : p.stages);
     volatile unsigned* const abort_flag = words + 1;
 
     const unsigned warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -133,10 +139,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     const int a_bufs = static_cast<int>(p.a_bufs);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; ++s) {
-            ptx::mbar_init(full_bar(s), 1);
-            ptx::mbar_init(empty_bar(s), W8 ? 5 : 1);  // the MMAs' commit; int8: and the four converter warps that read the raw box
-        }
+        for (int s = 0; s < fulls; ++s) ptx::mbar_init(full_bar(s), 1);
+        for (int s = 0; s < stages; ++s) ptx::mbar_init(empty_bar(s), W8 ? 5 : 1);  // the MMAs' commit; int8: and the four converter warps that read the raw box
         for (int s = 0; s < a_bufs; ++s) {
             ptx::mbar_init(a_full_bar(s), 4);
             ptx::mbar_init(a_empty_bar(s), 1);
@@ -158,33 +162,34 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     const uint32_t a_cols = tmem + n_tok;  // the weight buffers (64 columns a scale group) follow the accumulator
     ptx::grid_launch_dependents();
 
-    const auto load_w = [&](int i, int s) {
-        ptx::mbar_arrive_expect_tx(full_bar(s), stage + (W8 ? 256u : 0u));
-        ptx::tma_load_2d(base + s * stage, &map_w, full_bar(s), (k0 + i) * (W8 ? 128 : 64), static_cast<int>(row0));
-        if constexpr (W8) ptx::bulk_load(base + scale_off + s * 256, p.scales_t + static_cast<size_t>(k0 + i) * p.ld_st + row0, 256, full_bar(s));
+    const auto load_w = [&](int i, int s, int f) {
+        ptx::mbar_arrive_expect_tx(full_bar(f), stage + (W8 ? 256u : 0u));
+        ptx::tma_load_2d(base + s * stage, &map_w, full_bar(f), (k0 + i) * (W8 ? 128 : 64), static_cast<int>(row0));
+        if constexpr (W8) ptx::bulk_load(base + scale_off + s * 256, p.scales_t + static_cast<size_t>(k0 + i) * p.ld_st + row0, 256, full_bar(f));
     };
     const int early = p.early_w != 0 ? min(stages, iters) : 0;
     if (warp == 0 && lane == 0) {
-        for (int i = 0; i < early; ++i) load_w(i, i);
+        for (int i = 0; i < early; ++i) load_w(i, i, i);
     }
     ptx::grid_dependency_wait();
 
     if (warp == 0) {
         if (lane == 0) {
-            int s = 0;
+            int s = 0, f = 0;
             unsigned phase = 1;
             for (int i = 0; i < iters; ++i) {
                 if (i >= stages && !wait_barrier(empty_bar(s), phase, abort_flag, p.status, kStatusProducerEmpty)) {
                     grace_for_copies_in_flight();
                     break;
                 }
-                if (i >= early) load_w(i, s);
+                if (i >= early) load_w(i, s, f);
                 if constexpr (W8) {
-                    ptx::tma_load_2d(base + s * stage + kWBytes, &map_x, full_bar(s), (k0 + i) * 128, 0);
-                    ptx::tma_load_2d(base + s * stage + kWBytes + x_box, &map_x, full_bar(s), (k0 + i) * 128 + 64, 0);
+                    ptx::tma_load_2d(base + s * stage + kWBytes, &map_x, full_bar(f), (k0 + i) * 128, 0);
+                    ptx::tma_load_2d(base + s * stage + kWBytes + x_box, &map_x, full_bar(f), (k0 + i) * 128 + 64, 0);
                 } else {
-                    ptx::tma_load_2d(base + s * stage + kWBytes, &map_x, full_bar(s), (k0 + i) * 64, 0);
+                    ptx::tma_load_2d(base + s * stage + kWBytes, &map_x, full_bar(f), (k0 + i) * 64, 0);
                 }
+                if (++f == fulls) f = 0;
                 if (++s == stages) s = 0, phase ^= 1u;
             }
         }
@@ -192,12 +197,12 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     } else if (warp == 1) {
         if (lane == 0) {
             const uint32_t idesc = ptx::instr_desc_f16_f32acc(kRows, n_tok);
-            int s = 0, ab = 0;
+            int s = 0, f = 0, ab = 0;
             unsigned phase = 0, a_phase = 0;
             bool ok = true;
             for (int i = 0; i < iters; ++i) {
                 if ((W8 && !wait_barrier(a_full_bar(ab), a_phase, abort_flag, p.status, kStatusMmaConvFull)) ||
-                    !wait_barrier(full_bar(s), phase, abort_flag, p.status, kStatusMmaFull)) {
+                    !wait_barrier(full_bar(f), phase, abort_flag, p.status, kStatusMmaFull)) {
                     ok = false;
                     break;
                 }
@@ -216,7 +221,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 // a commit holds the issuing thread until its MMAs have drained: only where somebody waits for the slot
                 if (i + stages < iters) ptx::mma_commit(empty_bar(s));
                 if (W8 && i + a_bufs < iters) ptx::mma_commit(a_empty_bar(ab));
-                if (++s == stages) s = 0, phase ^= 1u;
+                if (++s == stages) s = 0;
+                if (++f == fulls) f = 0, phase ^= 1u;
                 if (W8 && ++ab == a_bufs) ab = 0, a_phase ^= 1u;
             }
             if (ok) ptx::mma_commit(acc_bar);
@@ -231,7 +237,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             const bool in_n = row0 + row < p.n;  // rows past N multiply by zero
             for (int i = static_cast<int>(set); i < iters; i += 2) {
                 const int s = i % stages, ab = i % a_bufs;
-                bool got = wait_barrier(full_bar(s), (i / stages) & 1, abort_flag, p.status, kStatusConvFull);
+                bool got = wait_barrier(full_bar(i % fulls), (i / fulls) & 1, abort_flag, p.status, kStatusConvFull);
                 if (got && i >= a_bufs) got = wait_barrier(a_empty_bar(ab), (i / a_bufs - 1) & 1, abort_flag, p.status, kStatusConvEmpty);
                 if (!__all_sync(0xFFFFFFFFu, got)) break;
                 ptx::tc_fence_after_sync();
