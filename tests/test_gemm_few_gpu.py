@@ -56,3 +56,24 @@ def test_few_rows_kernel(oracle, t, n, k, parts):
             # (1e-6 of the quotient form beside the sums' own error, which silu's slope of at most 1.1 and the product double)
             assert rel_fro(gated.cpu().numpy(), oracle.swiglu_packed(want, n // 2)) < 3 * tol
     ctx.close()
+
+
+@pytest.mark.parametrize("t,n,k,form", [(7, 6144, 2560, 5), (7, 2560, 9728, 8), (64, 9728, 2560, 3), (128, 4096, 4096, 4), (200, 2560, 4096, 6), (129, 4096, 2048, 4)])
+def test_automatic_parts_of_k_are_fixed(t, n, k, form):
+    """The parts of k, and with them the bits, are a function of the shape and the SM count (148): not of how a GPU's SMs lie in its GPCs."""
+    import torch
+
+    import sepal_runner_b200 as sb
+
+    ctx = sb.Context(0)
+    if ctx.info()["sm_count"] != 148:
+        pytest.skip("pinned for 148 SMs")
+    gen = torch.Generator(device="cuda").manual_seed(t + n)
+    x = torch.randn((t, k), generator=gen, device="cuda").half()
+    w = (torch.randn((n, k), generator=gen, device="cuda") * 0.05).half()
+    run = lambda config: ctx.gemm_f16(x, w, y_half=False, config=config)  # noqa: E731
+    auto = run(-1)
+    assert torch.equal(auto, run(1024 + form))
+    assert not torch.equal(auto, run(1024 + form - 1))
+    ctx.check_status()
+    ctx.close()
