@@ -104,7 +104,7 @@ void launch_gemm_w8g(Context& ctx, const void* x, std::size_t ld_x, const W8gMat
 
 /// Which kernel the automatic schedule (`config` -1) of launch_gemm_w8g gives a [t x k] by [n x k] multiply on a device of `sm_count`
 /// SMs: the tokens to a tile of the swapped kernel (96 to 192: one block; 256 or 320: two blocks of half as many), or 0 for the
-/// unswapped kernels. `staged`: the result leaves through shared memory and the TMA (16-byte aligned rows; every result but a float32
+/// others (unswapped, or the few-rows kernel). `staged`: the result leaves through shared memory and the TMA (16-byte aligned rows; every result but a float32
 /// SwiGLU and a binary16 residual update); `epilogue`: the SwiGLU's epilogue costs more, and a staged residual update with CTA pairs to
 /// spare has them share the tiles. Host arithmetic only.
 unsigned w8g_swapped_tokens(unsigned sm_count, std::size_t t, std::size_t n, std::size_t k, bool staged, Epilogue epilogue);

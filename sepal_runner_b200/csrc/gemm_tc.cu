@@ -2794,11 +2794,11 @@ void decode_config(int config, std::size_t n, bool coarse, bool auto_pair, const
 // 58 -> 28.3 / 32). From there to 256 rows where the cluster's parts of k still shorten the loop by more than its M of 128 rows loses:
 // four parts or more (200 rows: down 31.6 / 29.3 -> 17.7 / 19.2, k or v 15.1 / 14.7 -> 8.8 / 9.6), with fp16 weights two up to 208 rows
 // (qkv 16.7 -> 15.3; at 256 rows 16.8 against 17.8).
-bool few_rows_wins(const Context& ctx, const FewCall& call) {
-    if (call.t <= kBM) return true;
-    if (call.t > kFewMaxRows || call.k < 1024) return false;  // (a k loop of a dozen steps has nothing to share)
-    const unsigned split = few_schedule(static_cast<unsigned>(ctx.sm_count), call.t, call.n, call.k, call.int8).split;
-    return split >= 4 || (split >= 2 && !call.int8 && call.t <= 208);
+bool few_rows_wins(unsigned sm_count, std::size_t t, std::size_t n, std::size_t k, bool int8) {
+    if (t <= kBM) return true;
+    if (t > kFewMaxRows || k < 1024) return false;  // (a k loop of a dozen steps has nothing to share)
+    const unsigned split = few_schedule(sm_count, t, n, k, int8).split;
+    return split >= 4 || (split >= 2 && !int8 && t <= 208);
 }
 
 void launch_few(const Context& ctx, const FewCall& call, int config, cudaStream_t stream) {
@@ -2871,7 +2871,7 @@ void launch_gemm_f16(Context& ctx, const void* x, std::size_t ld_x, const void* 
     require_aligned(w, "W");
     check(cudaSetDevice(ctx.device), "cudaSetDevice");
     const FewCall few{x, ld_x, w, ld_w, false, nullptr, 0, nullptr, nullptr, y, ld_y, y_half, t, n, k, epilogue};
-    if (config >= kFewConfig || (config == -1 && few_rows_wins(ctx, few))) {
+    if (config >= kFewConfig || (config == -1 && few_rows_wins(static_cast<unsigned>(ctx.sm_count), t, n, k, false))) {
         launch_few(ctx, few, config, stream);
         return;
     }
@@ -2998,7 +2998,7 @@ void launch_gemm_f16(Context& ctx, const void* x, std::size_t ld_x, const void* 
 }
 
 unsigned w8g_swapped_tokens(unsigned sm_count, std::size_t t, std::size_t n, std::size_t k, bool staged, Epilogue epilogue) {
-    if (t > 0x7FFFFFFFu || n > 0x7FFFFFFFu || k > 0x7FFFFFFFu || k % kGroup != 0) return 0;
+    if (t > 0x7FFFFFFFu || n > 0x7FFFFFFFu || k > 0x7FFFFFFFu || k % kGroup != 0 || few_rows_wins(sm_count, t, n, k, true)) return 0;
     return pick_w8t_tokens(sm_count / 2, static_cast<unsigned>(t), static_cast<unsigned>(n), static_cast<unsigned>(k), staged,
                            epilogue == Epilogue::SwiGLU, epilogue == Epilogue::Add);
 }
@@ -3021,7 +3021,7 @@ void launch_gemm_w8g(Context& ctx, const void* x, std::size_t ld_x, const W8gMat
     check(cudaSetDevice(ctx.device), "cudaSetDevice");
     const bool padded_scales = unit_scales || (ld_st % 8 == 0 && ld_st >= (n + 127) / 128 * 128 && reinterpret_cast<std::uintptr_t>(scales_t) % 16 == 0);
     const FewCall few{x, ld_x, q, ld_q, true, scales_t, ld_st, descale, wm.col_scale, y, ld_y, y_half, t, n, k, epilogue};
-    if (config >= kFewConfig || (config == -1 && padded_scales && few_rows_wins(ctx, few))) {
+    if (config >= kFewConfig || (config == -1 && padded_scales && few_rows_wins(static_cast<unsigned>(ctx.sm_count), t, n, k, true))) {
         if (!padded_scales) throw std::invalid_argument("launch_gemm_w8g: scales_t must be 16-byte aligned with a row stride of at least N rounded up to 128");
         launch_few(ctx, few, config, stream);
         return;

@@ -123,3 +123,13 @@ def test_int8_schedule_query_is_host_arithmetic(lib):
     assert sb.w8g_schedule(0, 900, 2560, 9728, sb.ADD) == 0
     # the unhidden epilogue counts: a result stored lane by lane costs several us a wave more
     assert sb.w8g_schedule(148, 900, 4096, 2560, sb.STORE, staged=True) == 256 and sb.w8g_schedule(148, 900, 4096, 2560, sb.STORE, staged=False) == 0
+
+
+def test_int8_schedule_query_knows_the_few_rows_kernel(lib):
+    """Where the automatic choice is the few-rows kernel (up to 128 rows, and to 256 with k in four parts or more) the query does not name
+    the swapped kernel."""
+    import sepal_runner_b200 as sb
+
+    for t, n, k, want in ((1, 2560, 9728, 0), (129, 2560, 9728, 0), (200, 2560, 9728, 0), (200, 2560, 4096, 0), (200, 4096, 4096, 0),  # 20 to 32 tiles
+                          (200, 4352, 9728, 96), (200, 9728, 2560, 256), (257, 2560, 9728, 96), (200, 2560, 896, 96)):
+        assert sb.w8g_schedule(148, t, n, k, sb.STORE) == want, (t, n, k)
