@@ -408,18 +408,21 @@ void launch(const Context& ctx, const FewCall& c, FewSchedule sched, cudaStream_
 // Up to 64 rows: two CTAs to an SM, and as many parts of k as leave all clusters resident at once (a second wave, or a cluster that
 // waits for a GPC with room, costs more than the shorter k loop gives: 6144 x 2560, 7 rows: five parts 7.8 us, six 12.2). Up to 128 rows
 // a stage of the half-SM form is down to three or two slots, so a CTA with an SM to itself can be the better one: a k step costs about
-// 0.31 us there and 0.42 us, times the CTAs an SM has to feed, with two to an SM (fitted to twelve shapes). From 129 rows up one CTA to an SM.
+// 0.31 us there and 0.42 us, times the CTAs an SM has to feed, with two to an SM (fitted to twelve shapes of up to 148 tiles). Not with
+// more tiles than SMs: a second lone CTA starts when the first has ended, where two side by side hide one another's starts and ends (128
+// rows: 36864 x 1024 28.3 us alone, 21.9 as two; 65536 x 1024 54.0 and 40.1; 151936 x 2560 193 and 168). From 129 rows up one CTA to an SM.
 FewSchedule few_schedule(unsigned sm_count, std::size_t t, std::size_t n, std::size_t k, bool int8) {
     const std::size_t tiles = (n + kRows - 1) / kRows, iters = (k + (int8 ? 127 : 63)) / (int8 ? 128 : 64);
     FewSchedule best;
     double best_cost = 0.0;
-    for (unsigned slots = t <= 128 ? 2 : 1; slots >= (t <= 64 ? 2u : 1u); --slots) {
+    const unsigned most = t <= 128 ? 2u : 1u, least = t <= 64 || (t <= 128 && tiles > sm_count) ? 2u : 1u;
+    for (unsigned slots = most; slots >= least; --slots) {
         FewSchedule s;
         s.slots = slots;
         for (unsigned split = 2; split <= 8 && split <= iters; ++split)
             if (tiles <= slots * resident_clusters(sm_count, split)) s.split = split;
         const double steps = static_cast<double>((iters + s.split - 1) / s.split), load = static_cast<double>(tiles * s.split) / sm_count;
-        const double cost = steps * (slots == 2 ? 0.42 * (load > 1.0 ? load : 1.0) : 0.31 * (load > 1.0 ? 2.0 : 1.0));
+        const double cost = steps * (slots == 2 ? 0.42 * (load > 1.0 ? load : 1.0) : 0.31);
         if (best_cost == 0.0 || cost < best_cost) best = s, best_cost = cost;
     }
     return best;
