@@ -133,3 +133,6 @@ def test_int8_schedule_query_knows_the_few_rows_kernel(lib):
     for t, n, k, want in ((1, 2560, 9728, 0), (129, 2560, 9728, 0), (200, 2560, 9728, 0), (200, 2560, 4096, 0), (200, 4096, 4096, 0),  # 20 to 32 tiles
                           (200, 4352, 9728, 96), (200, 9728, 2560, 256), (257, 2560, 9728, 96), (200, 2560, 896, 96)):
         assert sb.w8g_schedule(148, t, n, k, sb.STORE) == want, (t, n, k)
+    # above 224 rows a float32 residual update needs five parts of k (26 tiles), not four (28)
+    assert sb.w8g_schedule(148, 224, 3584, 9728, sb.ADD) == 0 and sb.w8g_schedule(148, 225, 3328, 9728, sb.ADD) == 0
+    assert sb.w8g_schedule(148, 225, 3584, 9728, sb.ADD) != 0 and sb.w8g_schedule(148, 225, 3584, 9728, sb.STORE) == 0
