@@ -136,3 +136,21 @@ def test_int8_schedule_query_knows_the_few_rows_kernel(lib):
     # above 224 rows a float32 residual update needs five parts of k (26 tiles), not four (28)
     assert sb.w8g_schedule(148, 224, 3584, 9728, sb.ADD) == 0 and sb.w8g_schedule(148, 225, 3328, 9728, sb.ADD) == 0
     assert sb.w8g_schedule(148, 225, 3584, 9728, sb.ADD) != 0 and sb.w8g_schedule(148, 225, 3584, 9728, sb.STORE) == 0
+
+
+def test_current_stream_with_and_without_the_private_getter(lib, monkeypatch):
+    """The binding finds the current stream through torch's public functions where the private one is missing, and initialises CUDA as
+    they do (torch.cuda.current_device) where it is there."""
+    import types
+
+    import torch
+
+    from sepal_runner_b200 import lib as sbl
+
+    assert sbl._stream_ptr(types.SimpleNamespace(cuda_stream=5)) == 5
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=77))
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 1000 + device, raising=False)
+    assert sbl._stream_ptr(None) == 1003
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    assert sbl._stream_ptr(None) == 77
