@@ -3050,7 +3050,9 @@ void launch_gemm_w8g(Context& ctx, const void* x, std::size_t ld_x, const W8gMat
     const bool aligned_f32 = !y_half && reinterpret_cast<std::uintptr_t>(y) % 16 == 0 && ld_y % 4 == 0;
     const bool padded_scales = unit_scales || (ld_st % 8 == 0 && ld_st >= (n + 127) / 128 * 128 && reinterpret_cast<std::uintptr_t>(scales_t) % 16 == 0);
     const FewCall few{x, ld_x, q, ld_q, true, scales_t, ld_st, descale, wm.col_scale, y, ld_y, y_half, t, n, k, epilogue};
-    if (config >= kFewConfig || (config == -1 && padded_scales && few_rows_wins(static_cast<unsigned>(ctx.sm_count), t, n, k, true, epilogue, aligned_f32))) {
+    // (above 128 rows every other kernel wants rows padded to 256, as documented: one answer to a caller's table whatever the shape)
+    const bool few_padded = padded_scales && (t <= kBM || unit_scales || ld_st >= (n + 255) / 256 * 256);
+    if (config >= kFewConfig || (config == -1 && few_padded && few_rows_wins(static_cast<unsigned>(ctx.sm_count), t, n, k, true, epilogue, aligned_f32))) {
         if (!padded_scales) throw std::invalid_argument("launch_gemm_w8g: scales_t must be 16-byte aligned with a row stride of at least N rounded up to 128");
         launch_few(ctx, few, config, stream);
         return;

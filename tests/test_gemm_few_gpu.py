@@ -77,3 +77,24 @@ def test_automatic_parts_of_k_are_fixed(t, n, k, form):
     assert not torch.equal(auto, run(1024 + form - 1))
     ctx.check_status()
     ctx.close()
+
+
+def test_scale_rows_padded_to_128_only(oracle):
+    """Up to 128 rows such a table is taken; above, every shape refuses it, those of the few-rows kernel too."""
+    import torch
+
+    import sepal_runner_b200 as sb
+
+    ctx = sb.Context(0)
+    n, k = 384, 2048
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    q, s = ctx.quantize_group_s8(torch.randn((n, k), generator=gen, device="cuda"))
+    w = ctx.prepare_w8g(q, s)
+    short = sb.W8gWeight(q=q, scales=s, scales_t=w.scales_t[:, :n].contiguous(), descale=w.descale)
+    x = torch.randn((200, k), generator=gen, device="cuda").half()
+    assert torch.equal(ctx.gemm_w8g(x[:100], short), ctx.gemm_w8g(x[:100], w))
+    with pytest.raises(sb.SepalB200Error, match="rounded up to 256"):
+        ctx.gemm_w8g(x, short)
+    ctx.gemm_w8g(x, w)
+    ctx.check_status()
+    ctx.close()
