@@ -118,8 +118,8 @@ def test_more_runs_than_travel_with_the_launch(ctx):
 
 @pytest.mark.parametrize("value_heads,runs,length", [(4, 1, 100), (16, 2, 33), (32, 2, 49)])
 def test_layouts_agree(ctx, value_heads, runs, length):
-    """Bands at odd columns (channel by channel, value by value) give the bits of the same bands at aligned addresses (pairs, fours), whether a
-    block of the scan holds 16 columns of the state or more; tokens between the runs stay as they were."""
+    """Bands at odd columns (channel by channel, value by value) give the bits of the same bands at aligned addresses (pairs, fours), in blocks
+    of 16 columns of the state (the first case) and of 32; tokens between the runs stay as they were."""
     import torch
 
     import sepal_runner_b200 as sb
@@ -277,6 +277,41 @@ def test_output_on_the_inputs(ctx, value_heads, lengths, taps):
         got.append((out.clone(), st, tl))
     for x, y in zip(*got):
         assert torch.isfinite(x).all() and torch.equal(x, y)
+
+
+def test_column_blocks_agree(ctx):
+    """A request alone (sixteen columns of the state to a block of the scan: 16 heads are 128 blocks) gives the bits it gives among others
+    (32 columns), its state and tail too."""
+    import torch
+
+    import sepal_runner_b200 as sb
+
+    key_heads, value_heads, dim, lengths = 4, 16, 128, (57, 100, 16)
+    shape = sb.DeltaNetShape(key_heads=key_heads, value_heads=value_heads, head_dim=dim, conv_kernel=4, eps=1e-6)
+    assert value_heads * dim // 16 <= torch.cuda.get_device_properties(0).multi_processor_count < len(lengths) * value_heads * dim // 16
+    vd, cd = value_heads * dim, (2 * key_heads + value_heads) * dim
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    normal = lambda *s: torch.randn(s, generator=gen, device="cuda")  # noqa: E731
+    conv, a_log, dt_bias, norm = normal(cd, 4) * 0.5, normal(value_heads), normal(value_heads), 1 + normal(dim) * 0.1
+    states, tails = normal(len(lengths), value_heads, dim, dim) * 0.05, normal(len(lengths), 3, cd)
+    mixed, z, b, a = [normal(sum(lengths), w).half() for w in (cd, vd, value_heads, value_heads)]
+
+    def run(which):
+        begin = [sum(lengths[:i]) for i in range(len(lengths))]
+        tokens = torch.cat([torch.arange(begin[i], begin[i] + lengths[i]) for i in which]).cuda()
+        rows = [(sum(lengths[j] for j in which[:at]), lengths[i], i, 0) for at, i in enumerate(which)]
+        out = torch.empty((len(tokens), vd), dtype=torch.float16, device="cuda")
+        st, tl = states.clone(), tails.clone()
+        keep = sb.deltanet(ctx, shape, rows, mixed[tokens], z[tokens], b[tokens], a[tokens], conv, a_log, dt_bias, norm, st, tl, out)
+        ctx.check_status()
+        del keep
+        return out, st, tl, rows
+
+    out, st, tl, rows = run((0, 1, 2))
+    for i in range(len(lengths)):
+        alone = run((i,))
+        begin = rows[i][0]
+        assert torch.equal(alone[0], out[begin:begin + lengths[i]]) and torch.equal(alone[1][i], st[i]) and torch.equal(alone[2][i], tl[i])
 
 
 def test_arguments_are_checked(ctx):
