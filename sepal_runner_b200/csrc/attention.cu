@@ -825,6 +825,7 @@ void launch_attention_prepare(Context& ctx, const AttentionShape& shape, const A
     PrepareParams p{};
     for (std::size_t i = 0; i < shape.rotary_dims / 2; ++i) p.inv_freq[i] = std::pow(shape.rope_theta, -static_cast<double>(2 * i) / static_cast<double>(shape.rotary_dims));
     const std::size_t row_bytes = n_rows * sizeof(AttentionRow);
+    // (the angles are counted although they always travel with the launch: how many rows a call may have is a limit of the interface)
     char* table = table_memory(ctx, n_rows, (row_bytes + 15) / 16 * 16 + shape.rotary_dims / 2 * sizeof(double), n_rows <= kInlineRows);
     if (table == nullptr) {
         std::memcpy(p.near_rows, rows, row_bytes);

@@ -30,7 +30,7 @@ struct DeltaParams {
     unsigned char near_order[kInlineRuns];  // the runs, longest first
     unsigned n_rows, n_chunks;
     unsigned key_heads, value_heads, taps;
-    unsigned key_dim, value_dim, conv_dim;
+    unsigned value_dim, conv_dim;
     float eps;
     const void* mixed;
     const void* z;
@@ -779,6 +779,7 @@ void launch_deltanet(Context& ctx, const DeltaNetShape& shape, const DeltaNetRow
         chunks[i] = static_cast<unsigned>(n_chunks);
         n_chunks += (rows[i].length + kChunk - 1) / kChunk;
     }
+    // (what a call may have at most is counted as a row and 16 bytes a chunk, more than the table takes: a limit of the interface)
     const std::size_t rows_bytes = n_rows * sizeof(DeltaNetRow), table_bytes = rows_bytes + n_chunks * 16;
     if (ctx.table == nullptr || table_bytes > ctx.table_bytes / 2) throw std::invalid_argument("sepal_b200 deltanet: too many rows for the context's table");
     if (n_rows <= kInlineRuns) {
@@ -800,7 +801,6 @@ void launch_deltanet(Context& ctx, const DeltaNetShape& shape, const DeltaNetRow
     p.key_heads = shape.key_heads;
     p.value_heads = shape.value_heads;
     p.taps = shape.conv_kernel;
-    p.key_dim = shape.key_dim();
     p.value_dim = shape.value_dim();
     p.conv_dim = shape.conv_dim();
     p.eps = shape.eps;
@@ -831,8 +831,9 @@ void launch_deltanet(Context& ctx, const DeltaNetShape& shape, const DeltaNetRow
     p.out_stride = out_stride;
     const unsigned last = rows[n_rows - 1].q_begin + rows[n_rows - 1].length;
     p.n_tokens = last;
-    // two channels a load in the convolution, four values a load and store in the gated norm, where the types and addresses allow it
+    // (a limit of the interface: no kernel here holds more than 128 channels a warp)
     if (p.conv_dim > 40960) throw std::invalid_argument("sepal_b200 deltanet: the convolution is wider than 40960 channels");
+    // two channels a load in the convolution, four values a load and store in the gated norm, where the types and addresses allow it
     const bool pairs = mixed.half && shape.conv_kernel == 4 && mixed.stride % 2 == 0 && reinterpret_cast<std::uintptr_t>(mixed.data) % 4 == 0 &&
                        reinterpret_cast<std::uintptr_t>(weights.conv) % 16 == 0 && reinterpret_cast<std::uintptr_t>(tails) % 8 == 0;
     p.wide_norm = z.half && z.stride % 4 == 0 && reinterpret_cast<std::uintptr_t>(z.data) % 8 == 0 && out_stride % 4 == 0 && reinterpret_cast<std::uintptr_t>(out) % 8 == 0;

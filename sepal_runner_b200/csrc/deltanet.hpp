@@ -49,8 +49,8 @@ struct DeltaNetWeights {
 };
 
 /// Scratch of one call (device, float32, 16-byte aligned), sized for the call's tokens N: kq [key_heads, N, 264] (a token's k, q and 8
-/// floats of padding per key head); v, reads [N, value_dim]; coef [value_heads, N, 56] (the chunk coefficients); 2 N value_heads more that
-/// nothing uses.
+/// floats of padding per key head); v, reads [N, value_dim]; coef [value_heads, N, 56] (the chunk coefficients). The interface asks for
+/// 2 N value_heads more, which nothing uses, so that callers' sizes stay what they are.
 struct DeltaNetScratch {
     float* kq = nullptr;
     float* v = nullptr;
@@ -71,7 +71,7 @@ inline DeltaNetScratch deltanet_scratch(float* base, const DeltaNetShape& s, std
     return sc;
 }
 
-/// The launches of a layer (prepare with the chunk coefficients, scan, gated norm with the tails). mixed [N, conv_dim], z [N, value_dim], b and a [N, value_heads] are bands of the in-projection's output;
+/// The launches of a layer (prepare with the chunk coefficients, scan with the tails, gated norm). mixed [N, conv_dim], z [N, value_dim], b and a [N, value_heads] are bands of the in-projection's output;
 /// states float32 [slots, value_heads, head_dim, head_dim] and tails float32 [slots, K - 1, conv_dim], both updated in place; out
 /// binary16 [N, value_dim] with row stride out_stride.
 /// `rows` is a HOST array sorted by q_begin.
