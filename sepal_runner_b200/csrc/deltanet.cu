@@ -152,9 +152,10 @@ __device__ __forceinline__ float4 input_pairs_before(const DeltaParams& p, const
 // 64 + 2 l and 65 + 2 l: eleven rows are read for eight tokens, all in flight at once, and the taps once. `Pairs`: binary16 inputs and
 // four taps at addresses that allow two channels a load; otherwise channel by channel.
 //
-// What bounds it is instructions (61 % of the issue slots, the shared-memory pipe at 41 %): five runs of 2500 tokens in all, 32 value
-// heads, 69 us, where the convolution and the coefficients as two launches, with q and k written and read back between them, took
-// 74 + 65 us under the profiler. Four blocks to an SM hide one another's barriers (4096 tokens: 98 us, 104 with three).
+// What bounds it is instructions (71 % of the issue slots, the shared-memory pipe at 49 %): 4096 tokens of 32 value heads 116 us under the
+// profiler (95 with an approximate quotient in the sigmoid and 1 / norm multiplied, which gives other bits). The convolution and the
+// coefficients as two launches, with q and k written and read back between them, took 74 + 65 us for five runs of 2500 tokens in all,
+// where one launch took 69. Four blocks to an SM hide one another's barriers (4096 tokens: 98 us against 104 with three, then).
 constexpr int kHeadsAtOnce = 2;
 
 template <bool Pairs>
@@ -429,7 +430,7 @@ __device__ __forceinline__ void leave_tail(const DeltaParams& p, const DeltaNetR
 // v). The reads go to global memory in float32; the gated norm over a head's 128 reads is the next launch.
 //
 // One run, 32 value heads: 0.86 us a chunk, 54 ns a token (with one warp to sixteen columns 82 ns), and that is the latency of the chain:
-// the same without any copies, issue slots 38 %, tensor pipe 20 %, shared-memory pipe 41 %. Parts 2 and sixteen columns to a warp were
+// the same without any copies, issue slots 38 %, tensor pipe 23 %, shared-memory pipe 45 %. Parts 2 and sixteen columns to a warp were
 // the best of ten layouts (900 tokens: 53 us; four parts 63; one set of two by two 66; 64 columns to a block 78). Fetching the last
 // product's operands in the middle of the first products gave 9 %; 16-byte loads of k and q (fewer instructions) lost 5 %.
 //
@@ -693,8 +694,8 @@ void launch_scan(const Context& ctx, const DeltaParams& p, cudaStream_t stream) 
 
 // The gated norm of every token's and value head's 128 reads: x / sqrt(mean(x^2) + eps) * weight * silu(z) (the weight itself, not
 // 1 + weight). A warp takes four (token, head) pairs in a row, all their loads in flight together; lane l holds reads 4 l to 4 l + 3;
-// squares by fused multiply-add in that order, a butterfly. 4096 tokens, 32 heads, 134 MB: 45 us, bound by instructions (53 with the
-// divisions of a 64-bit unit number).
+// squares by fused multiply-add in that order, a butterfly. 4096 tokens, 32 heads, 134 MB: 50 us under the profiler, bound by
+// instructions (62 % of the issue slots).
 constexpr unsigned kNormUnits = 4;
 
 __global__ void __launch_bounds__(256) deltanet_norm_kernel(const __grid_constant__ DeltaParams p) {

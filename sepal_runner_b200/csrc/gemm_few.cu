@@ -2,11 +2,12 @@
 //
 // With T rows a weight of two bytes is worth 2 T operations, so below about 250 rows (half that for int8 weights) the multiply is bound
 // by reading W once. The kernels in gemm_tc.cu give a CTA 128 rows of X whatever T is and split N in wide tiles: a 7-row multiply by
-// 6144 x 2560 weights ran on 24 or 48 CTAs with 40 k steps each, 15.9 us for 31 MB. Here
+// 6144 x 2560 weights ran on 24 or 48 CTAs with 40 k steps each, 17.9 us for 31 MB; here 7.8 us behind one like it (alone under the profiler
+// 13 us, 30 % of the DRAM's throughput: a launch's start, its cluster's exchange and its end are the rest). Here
 //   - the weights are the MMA's first operand (128 rows of W to a CTA) and the tokens its second (N = T rounded up to 16), so nothing is
 //     computed for rows that are not there;
-//   - the k range of a tile of W is cut over the CTAs of a cluster (`split`, up to eight), so that about every SM streams its part of W
-//     whatever N is, and the parts meet through distributed shared memory in the order of their ranges: no scratch in global memory, no
+//   - the k range of a tile of W is cut over the CTAs of a cluster (`split`, up to eight), so that ceil(N / 128) split CTAs stream their
+//     parts of W (every SM from about 2300 rows of W on; 64 CTAs at 1024), and the parts meet through distributed shared memory in the order of their ranges: no scratch in global memory, no
 //     counters, the same bits every time;
 //   - a CTA takes at most half of an SM up to 64 rows: with the weights static the next multiply's CTAs are resident and have
 //     their first boxes of W requested while this one still drains.

@@ -142,8 +142,9 @@ void B200Gemm::gemm_f(const void* x, HostType type, std::size_t t, WeightId id, 
     float* dy = static_cast<float*>(scratch(t * w.n * 4, top));
     float* tmp = type == HostType::F16 ? nullptr : static_cast<float*>(scratch(t * w.k * 4, top));
     // The rows of a large call go through in up to kChunks pieces on three streams, so that the upload of piece i + 1, the multiply of
-    // piece i and the download of piece i - 1 run at the same time (the bus carries both directions at once). The multiplies of all
-    // pieces run on one stream, one after another: they share the context's split-k scratch.
+    // piece i and the download of piece i - 1 run at the same time (the bus carries both directions at once): with pinned host memory. A
+    // copy to pageable memory returns when it is done, so there the next piece is not enqueued before this one is down. The multiplies of
+    // all pieces run on one stream, one after another: they share the context's split-k scratch.
     constexpr std::size_t kChunks = 4, kMinChunk = 256;
     std::size_t pieces = t / kMinChunk;
     pieces = pieces < 1 ? 1 : (pieces > kChunks ? kChunks : pieces);
